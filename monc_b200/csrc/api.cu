@@ -204,6 +204,7 @@ static void fill_scalars(mgpu_handle* h) {
   s.coriolis = c.coriolis_enabled; s.surface_bcs = c.use_surface_boundary_conditions;
   s.use_vd = c.use_viscosity_and_diffusion;
   s.tvd_flow = c.advection_flow_fields == MGPU_ADVECT_TVD ? 1 : 0;
+  s.krylov = c.solver == MGPU_SOLVER_ITERATIVE ? 1 : 0;
   s.rho_unity = 1;
   for (int k = 1; k <= c.nz; ++k)
     if (r.rho[k] != 1.0 || r.rhon[k] != 1.0) s.rho_unity = 0;
@@ -255,6 +256,7 @@ static const std::vector<double>* prof_vec(const RefState& r, int id) {
     case P_TOFF: return &r.moist_toff; case P_TC0: return &r.tc0; case P_DZ: return &r.dz;
     case P_DMPCO: return &r.dmpco; case P_DMPCOZ: return &r.dmpcoz; case P_WSUBS: return &r.w_subs;
   }
+  if (id >= P_TVC1P && id < P_ALL) return &r.tvc[id - P_TVC1P];
   return nullptr;
 }
 
@@ -289,8 +291,8 @@ int mgpu_create(const mgpu_config* cfg, mgpu_handle** out) {
   if (cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking) != cudaSuccess) { delete h; return MGPU_ERR_CUDA; }
   // profiles
   const int stride = cfg->nz + 2;
-  std::vector<double> prof((size_t)P_COUNT * stride, 0.0);
-  for (int id = 0; id < P_COUNT; ++id) {
+  std::vector<double> prof((size_t)P_ALL * stride, 0.0);
+  for (int id = 0; id < P_ALL; ++id) {
     const std::vector<double>* v = prof_vec(h->rs, id);
     for (int k = 0; k <= cfg->nz && k < (int)v->size(); ++k) prof[(size_t)id * stride + k] = (*v)[k];
   }

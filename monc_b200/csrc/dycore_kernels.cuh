@@ -921,6 +921,9 @@ __global__ void __launch_bounds__(tiled::NT, tiled::ctas_momentum<T>()) k_f_mome
   }
 }
 
+// ---- TVD kernels of the separately rounded build and of models with the iterative solver (the
+// contracted build's others: tvd_fast.cuh) ------------------------------------------------------
+
 // One scalar of the centred step: `zf` is advected and diffused; with `src` null the kernel also
 // steps it (stepfields + the Robert pre-smoothing of swap_smooth, with the negative clip for q
 // fields) into out_f / out_zf, otherwise it writes the source (levels 2..nz) for the cloud step.
@@ -1744,6 +1747,47 @@ static int launch_moist(const Scalars& s, DevState<T>& d, int tiles, int nsm, in
   return 1;
 }
 
+// the scalars of the centred step: theta alone, theta with vapour and liquid in one pass (sources,
+// cloud and stepping included), or one launch per scalar writing its source, then saturation
+// adjustment and stepping
+template <typename T>
+static int launch_scalar_part(const Scalars& s, DevState<T>& d, int tiles, int nsm, int levels, cudaStream_t st) {
+  if (s.nq == 2) return launch_moist<T>(s, d, tiles, nsm, levels, st);
+  const size_t sm_s = tiled::scalar_smem<T>();
+  static int occ_s = 0;
+  if (!occ_s) {
+    cudaFuncSetAttribute(k_f_scalar_tiled<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_s);
+    cudaFuncSetAttribute(k_f_scalar_tiled<T>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_s, k_f_scalar_tiled<T>, tiled::NT, sm_s);
+    if (occ_s < 1) occ_s = 1;
+  }
+  const int nc_s = s.level_chunks > 0 ? s.level_chunks : choose_level_chunks(tiles, occ_s * nsm, levels, 0.002);
+  const int kc_s = (levels + nc_s - 1) / nc_s;
+  dim3 block(tiled::TX, tiled::TY, 1);
+  dim3 grid_s(s.nx / tiled::TX, s.ny / tiled::TY, (levels + kc_s - 1) / kc_s);
+  if (s.nq == 0) {
+    k_f_scalar_tiled<T><<<grid_s, block, sm_s, st>>>(s, d, kc_s, ScalarJob<T>{d.th, d.zth, d.th_n, d.zth_n, nullptr, 0, 2});
+    return 1;
+  }
+  k_f_scalar_tiled<T><<<grid_s, block, sm_s, st>>>(s, d, kc_s, ScalarJob<T>{d.th, d.zth, nullptr, nullptr, d.sth, 0, 2});
+  for (int n = 0; n < s.nq; ++n)
+    k_f_scalar_tiled<T><<<grid_s, block, sm_s, st>>>(s, d, kc_s, ScalarJob<T>{d.q[n], d.zq[n], nullptr, nullptr, d.sq[n], 1, 3 + n});
+  k_f_cloud_step<T><<<pt_grid(s, s.nz), pt_block(), 0, st>>>(s, d);
+  return s.nq + 2;
+}
+template <typename T>
+static int launch_flow_part(const Scalars& s, DevState<T>& d, int tiles, int nsm, int levels, cudaStream_t st) {
+  return launch_flow_tvd<T, 0>(s, d, d.su, tiles, nsm, levels, st) +
+         launch_flow_tvd<T, 1>(s, d, d.sv, tiles, nsm, levels, st) +
+         launch_flow_tvd<T, 2>(s, d, d.sw, tiles, nsm, levels, st);
+}
+}  // namespace KVARIANT
+}  // namespace mgpu
+#ifdef MGPU_CONTRACTED
+#include "tvd_fast.cuh"
+#endif
+namespace mgpu {
+namespace KVARIANT {
 // returns the number of kernels launched; `mid` (may be null) is recorded before the momentum kernel
 // returns the number of kernels launched
 template <typename T>
@@ -1786,54 +1830,43 @@ int launch_fused_dynamics(const Scalars& s, DevState<T>& d, cudaStream_t st, cud
     if (mid) cudaEventRecord(mid, st);
     return 1;
   }
-  const size_t sm_m = tiled::momentum_smem<T>(), sm_s = tiled::scalar_smem<T>();
-  static int occ_m = 0, occ_s = 0, nsm = 0;
+  const size_t sm_m = tiled::momentum_smem<T>();
+  static int occ_m = 0, nsm = 0;
   if (!nsm) {
     cudaFuncSetAttribute(k_f_momentum_tiled<T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_m);
     cudaFuncSetAttribute(k_f_momentum_tiled<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_m);
-    cudaFuncSetAttribute(k_f_scalar_tiled<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_s);
     cudaFuncSetAttribute(k_f_momentum_tiled<T, false>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
     cudaFuncSetAttribute(k_f_momentum_tiled<T, true>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
-    cudaFuncSetAttribute(k_f_scalar_tiled<T>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_m, k_f_momentum_tiled<T, false>, tiled::NT, sm_m);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_s, k_f_scalar_tiled<T>, tiled::NT, sm_s);
     int dev = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
     if (occ_m < 1) occ_m = 1;
-    if (occ_s < 1) occ_s = 1;
     if (nsm < 1) nsm = 1;
   }
   const int tiles = (s.nx / tiled::TX) * (s.ny / tiled::TY), levels = s.nz - 1;
-  const int nc_s = s.level_chunks > 0 ? s.level_chunks : choose_level_chunks(tiles, occ_s * nsm, levels, 0.002);
-  const int nc_m = s.level_chunks > 0 ? s.level_chunks : choose_level_chunks(tiles, occ_m * nsm, levels);
-  const int kc_s = (levels + nc_s - 1) / nc_s, kc_m = (levels + nc_m - 1) / nc_m;
-  dim3 block(tiled::TX, tiled::TY, 1);
-  dim3 grid_s(s.nx / tiled::TX, s.ny / tiled::TY, (levels + kc_s - 1) / kc_s);
-  dim3 grid_m(s.nx / tiled::TX, s.ny / tiled::TY, (levels + kc_m - 1) / kc_m);
-  int nscal = moist ? s.nq + 2 : 1;  // launches of the scalar part
-  if (!moist) {
-    k_f_scalar_tiled<T><<<grid_s, block, sm_s, st>>>(s, d, kc_s, ScalarJob<T>{d.th, d.zth, d.th_n, d.zth_n, nullptr, 0, 2});
-  } else if (s.nq == 2) {
-    // theta, vapour and liquid in one pass, sources, cloud and stepping included
-    nscal = launch_moist<T>(s, d, tiles, nsm, levels, st);
-  } else {
-    // one launch per scalar writing its source, then saturation adjustment and stepping
-    k_f_scalar_tiled<T><<<grid_s, block, sm_s, st>>>(s, d, kc_s, ScalarJob<T>{d.th, d.zth, nullptr, nullptr, d.sth, 0, 2});
-    for (int n = 0; n < s.nq; ++n)
-      k_f_scalar_tiled<T><<<grid_s, block, sm_s, st>>>(s, d, kc_s, ScalarJob<T>{d.q[n], d.zq[n], nullptr, nullptr, d.sq[n], 1, 3 + n});
-    k_f_cloud_step<T><<<pt_grid(s, s.nz), pt_block(), 0, st>>>(s, d);
-  }
+  int nl = 0;
+#ifdef MGPU_CONTRACTED
+  const bool contracted = !s.krylov;
+  if (contracted) nl += tvdf::launch_all_scalars<T>(s, d, st);
+#else
+  constexpr bool contracted = false;
+#endif
+  if (!contracted) nl += launch_scalar_part<T>(s, d, tiles, nsm, levels, st);
   if (mid) cudaEventRecord(mid, st);
-  int flow = 0;
   if (s.tvd_flow) {
-    flow += launch_flow_tvd<T, 0>(s, d, d.su, tiles, nsm, levels, st);
-    flow += launch_flow_tvd<T, 1>(s, d, d.sv, tiles, nsm, levels, st);
-    flow += launch_flow_tvd<T, 2>(s, d, d.sw, tiles, nsm, levels, st);
+#ifdef MGPU_CONTRACTED
+    if (contracted) nl += tvdf::launch_all_flow<T>(s, d, st);
+#endif
+    if (!contracted) nl += launch_flow_part<T>(s, d, tiles, nsm, levels, st);
   }
+  const int nc_m = s.level_chunks > 0 ? s.level_chunks : choose_level_chunks(tiles, occ_m * nsm, levels);
+  const int kc_m = (levels + nc_m - 1) / nc_m;
+  dim3 block(tiled::TX, tiled::TY, 1);
+  dim3 grid_m(s.nx / tiled::TX, s.ny / tiled::TY, (levels + kc_m - 1) / kc_m);
   if (s.tvd_flow) k_f_momentum_tiled<T, true><<<grid_m, block, sm_m, st>>>(s, d, kc_m);
   else k_f_momentum_tiled<T, false><<<grid_m, block, sm_m, st>>>(s, d, kc_m);
-  return nscal + 1 + flow;
+  return nl + 1;
 }
 template <typename T>
 void launch_fused_pressure_source(const Scalars& s, DevState<T>& d, cudaStream_t st) {

@@ -223,6 +223,21 @@ void build_reference_state(const mgpu_config& c, RefState& rs) {
     for (int k = 1; k <= n; ++k) rs.tc0[k] = rs.thref[k] * rs.rprefrcp[k] - 273.15;
     for (int k = 1; k <= n - 1; ++k) rs.moist_toff[k] = rs.rprefrcp[k] * rs.thref[k + 1] - rs.tstarpr[k] - rs.tref[k];
   }
+  // The vertical TVD face's curvature term (calculate_flux_in_w) is (1 - cfl^2)/6 dd^2 rdc ((fd - fc)
+  // rdd - (fc - fu) rdu): its coefficients of fd - fc and fc - fu over 1 - cfl^2, from the metrics
+  // of scalars, u, v (rdz, rdzn, dzn) and of w (rdzn, rdz, dz, the central rdz one level up)
+  for (auto& v : rs.tvc) v.assign(n + 2, 0.0);
+  for (int k = 1; k <= n - 1; ++k) {
+    const int k1 = k + 1, k2 = std::min(k + 2, n);
+    auto set = [&](int row, double dd, double rdc, double rdu) {
+      rs.tvc[row][k] = dd * rdc / 6.0;
+      rs.tvc[row + 1][k] = dd * dd * rdc * rdu / 6.0;
+    };
+    set(0, rs.dzn[k1], rs.rdz[k], rs.rdzn[k]);
+    set(2, rs.dzn[k1], rs.rdz[k1], rs.rdzn[k2]);
+    set(4, rs.dz[k1], rs.rdzn[k1], rs.rdz[k]);
+    set(6, rs.dz[k1], rs.rdzn[k2], rs.rdz[k2]);
+  }
   // neutral mixing length (gridmanager.F90:2298-2310)
   for (int k = 2; k <= n - 1; ++k) {
     rs.rneutml[k] = std::sqrt(1.0 / (1.0 / sqr(c.von_karman_constant * (rs.z[k] + c.z0)) + 1.0 / sqr(rs.rmlmax)));

@@ -18,6 +18,9 @@ struct RefState {
   std::vector<double> z, zn, dz, dzn, rdz, rdzn, rho, rhon, thref, dthref, czb, cza, czg, czh, tzc1, tzc2, tzd1, tzd2;
   std::vector<double> rneutml, rneutml_sq, buoy_co, prefn, prefrcp, rprefrcp, tref, tstarpr, qsat, dqsatdt, qsatfac;
   std::vector<double> gwx, gwy;  // geostrophic wind profile
+  // coefficients of the curvature term of the TVD face above level k, for upward (1P, 2P) and
+  // downward flow (1N, 2N), of scalars, u and v (rows 0..3) and of w (rows 4..7)
+  std::vector<double> tvc[8];
   std::vector<double> moist_toff, tc0;  // FP64 offsets of the FP32-mixed moist terms (grid.cpp)
   double czn = 0, zlogm = 0, zlogth = 0, vk_on_zlogm = 0;
   double dx = 0, dy = 0, cx = 0, cy = 0, cx2 = 0, cy2 = 0, tcx = 0, tcy = 0;
@@ -50,7 +53,10 @@ int checkpoint_read_host(const mgpu_config& c, const std::string& path, double* 
 enum ProfileId {
   P_RDZ = 0, P_RDZN, P_DZN, P_RHO, P_RHON, P_DTHREF, P_CZB, P_CZA, P_CZG, P_CZH, P_TZC1, P_TZC2, P_TZD1, P_TZD2,
   P_RNEUTML_SQ, P_BUOY_CO, P_THREF, P_PREFRCP, P_RPREFRCP, P_TREF, P_TSTARPR, P_QSAT, P_DQSATDT, P_QSATFAC,
-  P_GWX, P_GWY, P_PREFN, P_TOFF, P_TC0, P_DZ, P_DMPCO, P_DMPCOZ, P_WSUBS, P_COUNT
+  P_GWX, P_GWY, P_PREFN, P_TOFF, P_TC0, P_DZ, P_DMPCO, P_DMPCOZ, P_WSUBS, P_COUNT,
+  // the vertical TVD faces' metric products (RefState::tvc), read by the contracted build's kernels
+  // only and not staged with the P_COUNT profiles above
+  P_TVC1P = P_COUNT, P_TVC2P, P_TVC1N, P_TVC2N, P_TWC1P, P_TWC2P, P_TWC1N, P_TWC2N, P_ALL
 };
 
 // Scalars every dynamical-core kernel reads (passed by value as a kernel parameter).
@@ -71,11 +77,15 @@ struct Scalars {
   int point_dynamics;  // 1: always use the untiled dynamics kernel (MGPU_POINT_DYNAMICS=1)
   int level_chunks;    // level chunks of the tiled dynamics kernels; 0 = chosen from the occupancy
                        // (MGPU_LEVEL_CHUNKS=n fixes it)
+  int krylov;          // 1: the pressure solver is iterative.  Its iterates amplify rounding (a cold solve of
+                       // some hundred iterations turns 1e-14 in the source into 3e-3 in the pressure it
+                       // stops at), so the contracted build keeps to one set of kernels, the ones it
+                       // shares with the separately rounded build, for these models
   int rho_unity;       // 1 when rho = rhon = 1 on every level (Boussinesq with rhobous = 1)
   int passive_th, passive_q, nq, iqv, iql;
   int coriolis, surface_bcs, use_vd;
   int tvd_flow;            // 1: u, v, w advected by TVD (advection_flow_fields = tvd) instead of PW
-  const double* prof;      // device: P_COUNT profiles, each (nz+2) long, 1-based
+  const double* prof;      // device: P_ALL profiles, each (nz+2) long, 1-based
   const double* bmean;     // FP32-mixed fused step: horizontal means of th (row 0) and q(n) (row 1+n) per
                            // level, (nz+2) per row, removed from the buoyancy; null elsewhere
   const double* lookup;    // device: lookup_ustr, 1-based
