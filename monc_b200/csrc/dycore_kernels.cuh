@@ -1785,6 +1785,7 @@ static int launch_flow_part(const Scalars& s, DevState<T>& d, int tiles, int nsm
 }  // namespace mgpu
 #ifdef MGPU_CONTRACTED
 #include "tvd_fast.cuh"
+#include "momentum_fast.cuh"
 #endif
 namespace mgpu {
 namespace KVARIANT {
@@ -1820,8 +1821,17 @@ int launch_fused_subgrid(const Scalars& s, DevState<T>& d, cudaStream_t st) {
 }
 template <typename T>
 int launch_fused_dynamics(const Scalars& s, DevState<T>& d, cudaStream_t st, cudaEvent_t mid) {
-  // the tiled kernels cover centred dry steps; the first (forward) step and moist runs use the
-  // point kernel
+#ifdef MGPU_CONTRACTED
+  // centred steps, any horizontal size
+  if (!s.forward && !s.point_dynamics && !s.krylov && (!s.tvd_flow || (d.su && d.sv && d.sw))) {
+    int n = tvdf::launch_all_scalars<T>(s, d, st);
+    if (mid) cudaEventRecord(mid, st);
+    if (s.tvd_flow) n += tvdf::launch_all_flow<T>(s, d, st);
+    return n + momf::launch<T>(s, d, st);
+  }
+#endif
+  // the tiled kernels cover centred steps on sizes their tiles divide; the first (forward) step and
+  // other sizes use the point kernel
   const bool moist = s.nq > 0;
   const bool tiled_ok = !s.forward && !s.point_dynamics && (s.nx % tiled::TX) == 0 && (s.ny % tiled::TY) == 0 &&
                         s.nz >= 4 && (!moist || (d.sth && d.sq[s.nq - 1])) && (!s.tvd_flow || (d.su && d.sv && d.sw));
@@ -1845,21 +1855,9 @@ int launch_fused_dynamics(const Scalars& s, DevState<T>& d, cudaStream_t st, cud
     if (nsm < 1) nsm = 1;
   }
   const int tiles = (s.nx / tiled::TX) * (s.ny / tiled::TY), levels = s.nz - 1;
-  int nl = 0;
-#ifdef MGPU_CONTRACTED
-  const bool contracted = !s.krylov;
-  if (contracted) nl += tvdf::launch_all_scalars<T>(s, d, st);
-#else
-  constexpr bool contracted = false;
-#endif
-  if (!contracted) nl += launch_scalar_part<T>(s, d, tiles, nsm, levels, st);
+  int nl = launch_scalar_part<T>(s, d, tiles, nsm, levels, st);
   if (mid) cudaEventRecord(mid, st);
-  if (s.tvd_flow) {
-#ifdef MGPU_CONTRACTED
-    if (contracted) nl += tvdf::launch_all_flow<T>(s, d, st);
-#endif
-    if (!contracted) nl += launch_flow_part<T>(s, d, tiles, nsm, levels, st);
-  }
+  if (s.tvd_flow) nl += launch_flow_part<T>(s, d, tiles, nsm, levels, st);
   const int nc_m = s.level_chunks > 0 ? s.level_chunks : choose_level_chunks(tiles, occ_m * nsm, levels);
   const int kc_m = (levels + nc_m - 1) / nc_m;
   dim3 block(tiled::TX, tiled::TY, 1);

@@ -66,6 +66,14 @@ def test_level_chunks(gpu_lib, monkeypatch, flow, chunks, precision):
     compare((32, 8, 17), 0, False, precision, flow, chunks, monkeypatch)
 
 
+@pytest.mark.parametrize("precision", [cf.FP64, cf.FP32_MIXED], ids=["fp64", "fp32"])
+@pytest.mark.parametrize("grid", [(4, 4, 5), (30, 10, 9), (36, 20, 12), (50, 8, 7), (100, 60, 11)], ids=str)
+@pytest.mark.parametrize("nq,flow", [(2, cf.ADVECT_PW), (0, cf.ADVECT_TVD)], ids=["moist", "tvd"])
+def test_grids_no_tile_divides(gpu_lib, nq, flow, grid, precision):
+    """Tiles reaching past the domain; in FP32 nx = 30, 50 also rows that are not whole 16-byte chunks."""
+    compare(grid, nq, nq > 0, precision, flow)
+
+
 @pytest.mark.parametrize("flow", [cf.ADVECT_PW, cf.ADVECT_TVD], ids=["pw", "tvd"])
 def test_smallest_columns(gpu_lib, flow):
     compare((32, 8, 4), 0, False, cf.FP64, flow)
