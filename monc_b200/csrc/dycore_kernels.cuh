@@ -1786,6 +1786,7 @@ static int launch_flow_part(const Scalars& s, DevState<T>& d, int tiles, int nsm
 #ifdef MGPU_CONTRACTED
 #include "tvd_fast.cuh"
 #include "momentum_fast.cuh"
+#include "smag_fast.cuh"
 #endif
 namespace mgpu {
 namespace KVARIANT {
@@ -1793,6 +1794,9 @@ namespace KVARIANT {
 // returns the number of kernels launched
 template <typename T>
 int launch_fused_subgrid(const Scalars& s, DevState<T>& d, cudaStream_t st) {
+#ifdef MGPU_CONTRACTED
+  if (!s.point_dynamics && !s.krylov) return smagf::launch<T>(s, d, st);
+#endif
   const bool tiled_ok = !s.point_dynamics && (s.nx % tiled::TX) == 0 &&
                         (s.ny % tiled::TY) == 0 && s.nz >= 4;
   if (!tiled_ok) {
