@@ -39,7 +39,7 @@ constexpr int RL = 4;
 constexpr int RP = 3, RVIS = 4;
 template <typename T, bool TVD>
 constexpr size_t smem_bytes() {
-  return sizeof(T) * ((size_t)(6 * RP + RVIS) * G<T>::PLANE + (size_t)RL * L_N + (size_t)5 * CN);
+  return sizeof(T) * ((size_t)(6 * RP + RVIS) * G<T>::PLANE + (size_t)RL * L_N + (size_t)10 * CN);
 }
 template <typename T>
 constexpr int ctas() { return sizeof(T) == 4 ? 4 : 2; }
@@ -60,11 +60,9 @@ __global__ void __launch_bounds__(NT, ctas<T>()) k_f_momentum(const __grid_const
   T* const rL = rVIS + RVIS * PL;
   // the level's stresses: tau11, tau22 at the cells, tau12 at their upper right corners, tau13 and
   // tau23 on their right and upper sides
-  T* const t11 = rL + RL * L_N;
-  T* const t22 = t11 + CN;
-  T* const t12 = t22 + CN;
-  T* const t13 = t12 + CN;
-  T* const t23 = t13 + CN;
+  // (two buffers, alternating with the level: see the loop)
+  T* t11 = rL + RL * L_N;
+  T* t_next = t11 + 5 * CN;
   const int tid = threadIdx.x, tx = tid & 31, ty = tid >> 5;
   const int i0 = blockIdx.x * TX, j0 = blockIdx.y * TY;
   const int nz = s.nz;
@@ -104,7 +102,7 @@ __global__ void __launch_bounds__(NT, ctas<T>()) k_f_momentum(const __grid_const
       sg.copy(rVIS + (kk % RVIS) * PL, d.vis + lv);
     }
   };
-  for (int kk = kb; kk <= kb + 1 && kk <= nz; ++kk) stage(kk);
+  for (int kk = kb; kk <= kb + 2 && kk <= min(nz, ke + 1); ++kk) stage(kk);
   if (vd) sg.copy(rVIS + ((kb - 1) % RVIS) * PL, d.vis + (long long)(kb - 2) * plane);
   if (l_thread)
     for (int kk = kb; kk <= kb + 1 && kk <= nz; ++kk) rL[(kk & (RL - 1)) * L_N + tx] = level_const(kk);
@@ -168,22 +166,13 @@ __global__ void __launch_bounds__(NT, ctas<T>()) k_f_momentum(const __grid_const
   int s0 = (kb % RP) * PL, s1 = ((kb + 1) % RP) * PL, s2 = ((kb + 2) % RP) * PL;
   int vm_ = ((kb - 1) % RVIS) * PL, v0_ = (kb % RVIS) * PL, v1_ = ((kb + 1) % RVIS) * PL, v2_ = ((kb + 2) % RVIS) * PL;
   T u0 = rU[s0 + co], v0 = rV[s0 + co], w0 = rW[s0 + co];
+  T pnext = l_thread && kb + 2 <= min(nz, ke + 1) ? level_const(kb + 2) : (T)0.0;
   long long lev = lv0;
   for (int k = kb; k <= ke; ++k, lev += plane) {
-    if (k + 2 <= min(nz, ke + 1)) {
-      const long long lv = lev + 2 * plane;
-      sg.copy(rU + s2, d.u + lv);
-      sg.copy(rV + s2, d.v + lv);
-      sg.copy(rW + s2, d.w + lv);
-      if (vd) {
-        sg.copy(rZU + s2, d.zu + lv);
-        sg.copy(rZV + s2, d.zv + lv);
-        sg.copy(rZW + s2, d.zw + lv);
-        sg.copy(rVIS + v2_, d.vis + lv);
-      }
-    }
-    const bool pstage = l_thread && k + 2 <= min(nz, ke + 1);
-    const T pnext = pstage ? level_const(k + 2) : (T)0.0;
+    T *const t22 = t11 + CN, *const t12 = t22 + CN, *const t13 = t12 + CN, *const t23 = t13 + CN;
+    // (loaded a level ahead; level k+1 reads it after this level's barrier)
+    if (l_thread && k + 2 <= min(nz, ke + 1)) rL[((k + 2) & (RL - 1)) * L_N + tx] = pnext;
+    if (l_thread && k + 3 <= min(nz, ke + 1)) pnext = level_const(k + 3);
     const long long o = lev + col;
     const bool in = k < nz;
     const Raw raw = in ? load_raw(o + plane) : Raw{(T)0.0, (T)0.0, (T)0.0};
@@ -228,7 +217,8 @@ __global__ void __launch_bounds__(NT, ctas<T>()) k_f_momentum(const __grid_const
       su = su + f * ((T)0.25 * (vx + vxs) + (T)s.vgal - L[L_GWY]);
       sv = sv - f * ((T)0.25 * (uy + uym) + (T)s.ugal - L[L_GWX]);
     }
-    T zu = (T)0.0, zv = (T)0.0, zw = (T)0.0;
+    T zu = (T)0.0, zv = (T)0.0, zw = (T)0.0, va = (T)0.0, m11 = (T)0.0, m22 = (T)0.0, m12 = (T)0.0, m13 = (T)0.0,
+      m23 = (T)0.0, t33u = (T)0.0;
     if (vd) {
       const T *pZU = rZU + s0, *pZV = rZV + s0, *pZW = rZW + s0, *pA = rVIS + v0_, *pB = rVIS + vm_;
       // vis(k) + vis(k-1) of the cell at offset c, and the stresses of that cell
@@ -245,10 +235,15 @@ __global__ void __launch_bounds__(NT, ctas<T>()) k_f_momentum(const __grid_const
       zu = pZU[co];
       zv = pZV[co];
       zw = pZW[co];
-      const T va = vsum(co);
-      const T m11 = va * (zu - pZU[co - 1]) * cx, m22 = va * (zv - pZV[co - PW]) * cy;
-      const T m12 = tau12(co, (va + vsum(co + PW)) + (vsum(co + 1) + vsum(co + PW + 1)));
-      const T m13 = in ? tau13(co, zu) : (T)0.0, m23 = in ? tau23(co, zv) : (T)0.0;
+      va = vsum(co);
+      m11 = va * (zu - pZU[co - 1]) * cx;
+      m22 = va * (zv - pZV[co - PW]) * cy;
+      m12 = tau12(co, (va + vsum(co + PW)) + (vsum(co + 1) + vsum(co + PW + 1)));
+      if (in) {
+        m13 = tau13(co, zu);
+        m23 = tau23(co, zv);
+        t33u = (rVIS[v1_ + co] + pA[co]) * (rZW[s1 + co] - zw) * rL[((k + 1) & (RL - 1)) * L_N + L_RDZ];
+      }
       t11[own] = m11;
       t22[own] = m22;
       t12[own] = m12;
@@ -270,20 +265,36 @@ __global__ void __launch_bounds__(NT, ctas<T>()) k_f_momentum(const __grid_const
         const int c = (HY + tx) * PW + Gt::V + TX;
         t11[(tx + 1) * CW + TX + 1] = vsum(c) * (pZU[c] - pZU[c - 1]) * cx;
       }
-      __syncthreads();
+    } else if (act) {
+      zu = d.zu[o];
+      zv = d.zv[o];
+      zw = d.zw[o];
+    }
+    asm volatile("cp.async.wait_all;\n" ::: "memory");
+    __syncthreads();
+    // The stresses of the level are known, no plane of it is read below and level k+2 has landed: one
+    // barrier a level.  (A thread ahead writes the next level's stresses to the other buffer.)
+    if (k + 3 <= min(nz, ke + 1)) {
+      const long long lv = lev + 3 * plane;
+      sg.copy(rU + s0, d.u + lv);
+      sg.copy(rV + s0, d.v + lv);
+      sg.copy(rW + s0, d.w + lv);
+      if (vd) {
+        sg.copy(rZU + s0, d.zu + lv);
+        sg.copy(rZV + s0, d.zv + lv);
+        sg.copy(rZW + s0, d.zw + lv);
+        sg.copy(rVIS + vm_, d.vis + lv);
+      }
+    }
+    if (vd) {
       su = su + (t11[own + 1] - m11) * cx + (m12 - t12[own - CW]) * cy + (m13 - t13d) * L[L_RDZ];
       sv = sv + (m12 - t12[own - 1]) * cx + (t22[own + CW] - m22) * cy + (m23 - t23d) * L[L_RDZ];
       if (in) {
-        const T t33u = (rVIS[v1_ + co] + pA[co]) * (rZW[s1 + co] - zw) * rL[((k + 1) & (RL - 1)) * L_N + L_RDZ];
         sw = sw + (m13 - t13[own - 1]) * cx + (m23 - t23[own - CW]) * cy + (t33u - t33) * L[L_RDZN];
         t33 = t33u;
       }
       t13d = m13;
       t23d = m23;
-    } else if (act) {
-      zu = d.zu[o];
-      zv = d.zv[o];
-      zw = d.zw[o];
     }
     const T bhi = in ? buoyancy(k + 1, raw) : (T)0.0;
     if (in) sw = sw + (blo + bhi);
@@ -306,13 +317,13 @@ __global__ void __launch_bounds__(NT, ctas<T>()) k_f_momentum(const __grid_const
     u0 = uu; v0 = vu; w0 = wu;
     wxd = wx; wyd = wy;
     blo = bhi;
-    if (pstage) rL[((k + 2) & (RL - 1)) * L_N + tx] = pnext;
     int q = s0;
     s0 = s1; s1 = s2; s2 = q;
     q = vm_;
     vm_ = v0_; v0_ = v1_; v1_ = v2_; v2_ = q;
-    asm volatile("cp.async.wait_all;\n" ::: "memory");
-    __syncthreads();
+    T* const t = t11;
+    t11 = t_next;
+    t_next = t;
   }
 }
 
