@@ -21,11 +21,10 @@
 //  * the velocity part of a face is formed once for the NS fields;
 //  * the vertical metrics come as four ready coefficients per level (P_TVC1P ..).
 // Measured against the kernels of the separately rounded build's form (developed flow): theta at
-// 256 x 256 x 128 0.373 -> 0.277 ms in FP64 and 0.250 -> 0.166 ms in FP32; theta, vapour and liquid
-// at 512 x 512 x 160 5.78 -> 2.69 and 3.47 -> 1.42 ms; theta and five q fields at 1024 x 1024 x 200
-// in FP32 36.6 -> 13.0 ms; u, v, w at 256 x 256 x 128 in FP64 1.12 -> 0.67 ms.  FP64 moves 537 MB
-// for theta, 0.082 ms; what is left above that is issue (47% of slots with 16 warps per SM) and
-// the barriers between the faces and the sources of a level.
+// 256 x 256 x 128 0.373 -> 0.246 ms in FP64 and 0.250 -> 0.162 ms in FP32; theta, vapour and liquid
+// at 512 x 512 x 160 5.78 -> 2.54 and 3.47 -> 1.35 ms; theta and five q fields at 1024 x 1024 x 200
+// in FP32 36.6 -> 12.2 ms; u, v, w at 256 x 256 x 128 in FP64 1.12 -> 0.64 ms.  FP64 moves 537 MB
+// for theta, 0.082 ms; what is left above that is issue and latency with 16 warps per SM.
 #pragma once
 
 namespace mgpu {
@@ -60,11 +59,15 @@ struct Rings {
   static constexpr int UP = DIM == 2 ? 1 : 0;  // levels above k+1 the table of level k+1 reads
   static constexpr int RZ = 5, RF = 2 + UP, RD = DIM < 0 ? 3 : 0;
 };
+// Two copies of the face fluxes and cell tables, alternating with the level, make one barrier a level
+// do (theta, FP64, 256 x 256 x 128: 0.277 -> 0.246 ms); three FP64 fields leave no room for them at two CTAs.
+template <typename T, int NS>
+constexpr int copies() { return sizeof(T) == 8 && NS == 3 ? 1 : 2; }
 template <typename T, int NS, int DIM>
 constexpr size_t smem_bytes() {
   typedef Rings<DIM> R;
   return sizeof(T) * ((size_t)(NS * R::RZ + 3 * R::RF + R::RD) * G<T>::PLANE + (size_t)RL * L_N +
-                      (size_t)4 * CN + (size_t)NS * (TY * (TX + 1) + (TY + 1) * TX) + TX + TY);
+                      copies<T, NS>() * ((size_t)4 * CN + (size_t)NS * (TY * (TX + 1) + (TY + 1) * TX) + TX + TY));
 }
 // Resident CTAs the registers are sized for.  FP64 at two CTAs (no spills) runs faster than at
 // three with 80 registers and spills (0.292 against 0.326 ms for theta at 256 x 256 x 128); FP32
@@ -72,7 +75,7 @@ constexpr size_t smem_bytes() {
 // fields (1.48 against 1.64 ms at 512 x 512 x 160).
 template <typename T, int NS, int DIM>
 constexpr int ctas() {
-  if (sizeof(T) == 4) return NS == 1 ? 4 : 3;
+  if (sizeof(T) == 4) return NS == 1 && DIM != 2 ? 4 : 3;  // (w's dual grid takes more registers)
   return 2;
 }
 
@@ -179,13 +182,16 @@ struct PlaneStager {
   }
   // level pointer `lev` (the field's base plus whole levels) into the plane at `dst`
   __device__ __forceinline__ void copy(T* dst, const T* __restrict__ lev) const {
+    copy_to((unsigned)__cvta_generic_to_shared(dst + soff), lev + goff);
+  }
+  // the same with this thread's offsets (soff, goff) already in the two addresses
+  __device__ __forceinline__ void copy_to(unsigned a, const T* __restrict__ g) const {
     if (!on) return;
-    const unsigned a = (unsigned)__cvta_generic_to_shared(dst + soff);
     if (sizeof(T) == 4 && halves) {
-      asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(a), "l"(lev + goff) : "memory");
-      asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(a + 8), "l"(lev + goff2) : "memory");
+      asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(a), "l"(g) : "memory");
+      asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(a + 8), "l"(g + (goff2 - goff)) : "memory");
     } else {
-      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(a), "l"(lev + goff) : "memory");
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(a), "l"(g) : "memory");
     }
   }
 };
@@ -237,11 +243,12 @@ __global__ void __launch_bounds__(NT, ctas<T, NS, DIM>()) k_f_tvd(const __grid_c
   T* const rW = rV + R::RF * PL;
   T* const rD = rW + R::RF * PL;
   T* const rL = rD + R::RD * PL;                        // level constants
-  T2* const tVW = reinterpret_cast<T2*>(rL + RL * L_N); // cell tables of the level: (vs, ws) and (us, r)
-  T2* const tUR = tVW + CN;
-  T* const FX = reinterpret_cast<T*>(tUR + CN);         // NS x x-face fluxes of columns i0-1 .. i0+TX-1
-  T* const FY = FX + NS * NFX;                          // NS x y-face fluxes of rows j0-1 .. j0+TY-1
-  T* const BV = FY + NS * NFY;                          // v of the cells below the tile, u of those to its left
+  // of each copy: cell tables (vs, ws) and (us, r), NS x x-face fluxes of columns i0-1 .. i0+TX-1, NS x
+  // y-face fluxes of rows j0-1 .. j0+TY-1, v of the cells below the tile and u of those to its left
+  constexpr bool DB = copies<T, NS>() == 2;
+  constexpr int COPY = 4 * CN + NS * (NFX + NFY) + TX + TY;
+  T* cur = rL + RL * L_N;             // the copy of level k
+  T* nxt = DB ? cur + COPY : cur;     // and that of level k+1
   const int tid = threadIdx.x, lane = tid & 31;
   const int tx = lane, ty = tid >> 5;  // the warp's row
   const int i0 = blockIdx.x * TX, j0 = blockIdx.y * TY;
@@ -294,8 +301,10 @@ __global__ void __launch_bounds__(NT, ctas<T, NS, DIM>()) k_f_tvd(const __grid_c
 
   PlaneStager<T> sg;
   sg.init(s, j0, i0, tid);
+  T2 *tVW = reinterpret_cast<T2*>(cur), *tUR = tVW + CN;
+  T* BV = cur + 4 * CN + NS * (NFX + NFY);
   const int k0 = kb == 2 ? 1 : kb - 2;
-  // advected fields kb-2 .. kb+2 (level k in slot k mod RZ), flow kb+1 (.. kb+2), diff kb-1 .. kb
+  // advected fields kb-2 .. kb+2 (level k in slot k mod RZ), flow and diff as many as their rings hold
   for (int kk = k0; kk <= kb + 2 && kk <= nz; ++kk) {
     T* dst = rF + (kk % R::RZ) * PL;
     const long long lv = (long long)(kk - 1) * plane;
@@ -309,9 +318,9 @@ __global__ void __launch_bounds__(NT, ctas<T, NS, DIM>()) k_f_tvd(const __grid_c
     sg.copy(rV + o, job.v + lv);
     sg.copy(rW + o, job.w + lv);
   };
-  for (int kk = kb + 1; kk <= kb + 1 + R::UP && kk <= nz; ++kk) stage_flow(kk);
+  for (int kk = kb + 1; kk <= kb + 2 + R::UP && kk <= min(nz, ke + 1 + R::UP); ++kk) stage_flow(kk);
   if constexpr (DIM < 0)
-    for (int kk = kb - 1; kk <= kb; ++kk) sg.copy(rD + (kk % 3) * PL, job.diff + (long long)(kk - 1) * plane);
+    for (int kk = kb - 1; kk <= kb + 1 && kk <= ke; ++kk) sg.copy(rD + (kk % 3) * PL, job.diff + (long long)(kk - 1) * plane);
   if (l_thread)
     for (int kk = kb - 1; kk <= kb + 1 && kk <= nz; ++kk) rL[(kk & (RL - 1)) * L_N + lane] = level_const(kk);
   const T dtm_x2 = (T)dt_d;
@@ -419,27 +428,37 @@ __global__ void __launch_bounds__(NT, ctas<T, NS, DIM>()) k_f_tvd(const __grid_c
     fz_lo[0] = wlow * tvd_face_z_bottom<T, GF, View<T>, Prof<T>, TvdMetricW>(s, prof<T>(s), IU, IV, IW,
                                                                             view<T>(job.zf[0], s), dtm_x2, j, i);
   }
-  // the first prefetch overwrites the slot of level kb-2 that this face read
-  __syncthreads();
   int dm = ((kb - 1) % 3) * PL, d0 = (kb % 3) * PL, d1 = ((kb + 1) % 3) * PL;
-  int fo = ((kb + 1) % R::RF) * PL;  // slot of the flow at k+1
+  int fo = ((kb + 1) % R::RF) * PL;             // slot of the flow at k+1
   long long lev = (long long)(kb - 1) * plane;  // offset of level k
-  for (int k = kb; k <= ke; ++k, lev += plane) {
-    if (k + 3 <= min(nz, ke + 2)) {
+  const unsigned sa = (unsigned)__cvta_generic_to_shared(rF + sg.soff);
+  long long go = lev + sg.goff;
+  auto stage_field = [&](int slot, long long off) {
 #pragma unroll
-      for (int n = 0; n < NS; ++n) sg.copy(rF + n * R::RZ * PL + z3, job.zf[n] + lev + 3 * plane);
-    }
-    if (k + 2 + R::UP <= min(nz, ke + 1 + R::UP)) {
-      const long long lv = lev + (2 + R::UP) * plane;
-      const int o = R::UP ? ((k + 3) % R::RF) * PL : PL - fo;
-      sg.copy(rU + o, job.u + lv);
-      sg.copy(rV + o, job.v + lv);
-      sg.copy(rW + o, job.w + lv);
+    for (int n = 0; n < NS; ++n) sg.copy_to(sa + (unsigned)(sizeof(T) * (n * R::RZ * PL + slot)), job.zf[n] + off);
+  };
+  // when the planes of level k that its faces and cells read are free: field k+4 into the slot of k-1,
+  // flow k+3 into that of k+1 (w on its dual grid: one level up), diff k+2 into that of k-1
+  auto stage_next = [&](int k) {
+    if (k + 4 <= min(nz, ke + 2)) stage_field(zm, go + 4 * plane);
+    if (k + 3 + R::UP <= min(nz, ke + 1 + R::UP)) {
+      const long long off = go + (3 + R::UP) * plane;
+      const unsigned f = sa + (unsigned)(sizeof(T) * (NS * R::RZ * PL + fo));
+      sg.copy_to(f, job.u + off);
+      sg.copy_to(f + (unsigned)(sizeof(T) * R::RF * PL), job.v + off);
+      sg.copy_to(f + (unsigned)(sizeof(T) * 2 * R::RF * PL), job.w + off);
     }
     if constexpr (DIM < 0)
-      if (k + 1 <= ke) sg.copy(rD + d1, job.diff + lev + plane);
-    const bool pstage = l_thread && k + 2 <= min(nz, ke + 1);
-    const T pnext = pstage ? level_const(k + 2) : (T)0.0;
+      if (k + 2 <= ke) sg.copy_to(sa + (unsigned)(sizeof(T) * ((NS * R::RZ + 3 * R::RF) * PL + dm)), job.diff + go + 2 * plane);
+  };
+  // the slot of level kb-2, which the face below the chunk read, takes level kb+3
+  __syncthreads();
+  if (kb + 3 <= min(nz, ke + 2)) stage_field(z3, go + 3 * plane);
+  T pnext = l_thread && kb + 2 <= min(nz, ke + 1) ? level_const(kb + 2) : (T)0.0;
+  for (int k = kb; k <= ke; ++k, lev += plane, go += plane) {
+    // level constants of k+2, loaded a level ahead; level k+1 reads them after this level's barrier
+    if (l_thread && k + 2 <= min(nz, ke + 1)) rL[((k + 2) & (RL - 1)) * L_N + lane] = pnext;
+    if (l_thread && k + 3 <= min(nz, ke + 1)) pnext = level_const(k + 3);
     const long long o = lev + col;
     T fv[NS];
     if constexpr (DIM < 0) {
@@ -448,6 +467,9 @@ __global__ void __launch_bounds__(NT, ctas<T, NS, DIM>()) k_f_tvd(const __grid_c
     }
     const T* L = rL + (k & (RL - 1)) * L_N;
     const T* Ln = rL + ((k + 1) & (RL - 1)) * L_N;
+    T2 *const tVW = reinterpret_cast<T2*>(cur), *const tUR = tVW + CN;
+    T2 *const tVWn = reinterpret_cast<T2*>(nxt), *const tURn = tVWn + CN;
+    T *const FX = cur + 4 * CN, *const FY = FX + NS * NFX, *const BV = FY + NS * NFY, *const BVn = nxt + (BV - cur);
     if (DIM != 2 || k <= ktop) {
       const int fo2 = R::UP ? ((k + 2) % R::RF) * PL : 0;
       const bool top = k + 1 == nz;
@@ -491,6 +513,11 @@ __global__ void __launch_bounds__(NT, ctas<T, NS, DIM>()) k_f_tvd(const __grid_c
       Cell<T> cn{};
       T un = (T)0.0, vn = (T)0.0, wn = (T)0.0;
       if (k < nz) cn = next_cell(co, w0, un, vn, wn);
+      // the tables of level k+1: at once where they have a copy of their own
+      auto put_own = [&]() {
+        tVWn[own] = T2{cn.vs, cn.ws};
+        tURn[own] = T2{cn.us, cn.r};
+      };
       Cell<T> bn{};
       T bvn = (T)0.0;
       if (hr >= 0 && k < nz) {
@@ -498,6 +525,16 @@ __global__ void __launch_bounds__(NT, ctas<T, NS, DIM>()) k_f_tvd(const __grid_c
         bn = next_cell(bco, bw, bu, bv, bwn);
         bvn = hr == 0 ? bv : bu;
         bw = bwn;
+      }
+      auto put_border = [&]() {
+        tVWn[bcell] = T2{bn.vs, bn.ws};
+        tURn[bcell] = T2{bn.us, bn.r};
+        if (hr == 0) BVn[lane] = bvn;
+        if (hc == 0) BVn[TX + lane] = bvn;
+      };
+      if (DB && k < nz) {
+        put_own();
+        if (hr >= 0) put_border();
       }
       T fz_hi[NS];
 #pragma unroll
@@ -537,31 +574,10 @@ __global__ void __launch_bounds__(NT, ctas<T, NS, DIM>()) k_f_tvd(const __grid_c
         h_face(BV[TX + lane], cdx, cx, (lane + HY) * PW + Gt::V - 1, 1, PW, bvw.y + nvw.y, bvw.x + nvw.x, bur.y, tUR[o0 + 1].y,
                FX + lane * (TX + 1), NFX);
       }
-      __syncthreads();
-      // every face of the level is known and the cell tables are free for the next level's
-      if (k < nz) {
-        tVW[own] = T2{cn.vs, cn.ws};
-        tUR[own] = T2{cn.us, cn.r};
-        if (hr >= 0) {
-          tVW[bcell] = T2{bn.vs, bn.ws};
-          tUR[bcell] = T2{bn.us, bn.r};
-          if (hr == 0) BV[lane] = bvn;
-          if (hc == 0) BV[TX + lane] = bvn;
-        }
-      }
-      T src[NS];
-#pragma unroll
-      for (int n = 0; n < NS; ++n) {
-        const T* fx = FX + n * NFX + ty * (TX + 1) + tx;
-        const T* fy = FY + n * NFY + ty * TX + tx;
-        src[n] = ((fx[0] - fx[1]) + (fy[0] - fy[TX])) + (fz_lo[n] * L[L_T1] - fz_hi[n] * L[L_T2]);
-        fz_lo[n] = fz_hi[n];
-      }
-      if constexpr (DIM >= 0) {
-        if (act) job.src[o] = src[0];
-      } else {
+      // what of the source needs the planes: diffusion, damping, subsidence
+      T src[NS], zv[NS];
+      auto local_source = [&]() {
         if (job.first && s.th_baroclinic) src[0] = src[0] + ((v0 + (T)s.vgal) * (T)s.mfx - (u0 + (T)s.ugal) * (T)s.mfy);
-        T zv[NS];
         if (s.use_vd) {
           // diffusion_point, its level sums of the diffusivity formed once for the NS fields
           const T *pm = rD + dm + co, *p0 = rD + d0 + co;
@@ -598,6 +614,29 @@ __global__ void __launch_bounds__(NT, ctas<T, NS, DIM>()) k_f_tvd(const __grid_c
                              : subsidence_q_point<T>(s, P, F, job.row[n] - 3, k, j, i, src[n]);
           }
         }
+      };
+#pragma unroll
+      for (int n = 0; n < NS; ++n) src[n] = (T)0.0;
+      if constexpr (DB && DIM < 0) local_source();
+      if constexpr (DB) asm volatile("cp.async.wait_all;\n" ::: "memory");
+      __syncthreads();
+      // every face of the level is known
+      if constexpr (DB) stage_next(k);
+      if (!DB && k < nz) {
+        put_own();
+        if (hr >= 0) put_border();
+      }
+#pragma unroll
+      for (int n = 0; n < NS; ++n) {
+        const T* fx = FX + n * NFX + ty * (TX + 1) + tx;
+        const T* fy = FY + n * NFY + ty * TX + tx;
+        src[n] = src[n] + (((fx[0] - fx[1]) + (fy[0] - fy[TX])) + (fz_lo[n] * L[L_T1] - fz_hi[n] * L[L_T2]));
+        fz_lo[n] = fz_hi[n];
+      }
+      if constexpr (DIM >= 0) {
+        if (act) job.src[o] = src[0];
+      } else {
+        if constexpr (!DB) local_source();
         if constexpr (CLOUD) {
           // fields 1 and 2 are vapour and liquid
           const CloudProf<T> P{L, k, s};
@@ -619,7 +658,11 @@ __global__ void __launch_bounds__(NT, ctas<T, NS, DIM>()) k_f_tvd(const __grid_c
     } else {
       if (act) job.src[o] = (T)0.0;  // w at the top level
     }
-    if (pstage) rL[((k + 2) & (RL - 1)) * L_N + lane] = pnext;
+    if constexpr (!DB) {
+      asm volatile("cp.async.wait_all;\n" ::: "memory");
+      __syncthreads();
+      stage_next(k);
+    }
     // the planes move down a level
     const int zt = zm;
     zm = z0;
@@ -632,8 +675,9 @@ __global__ void __launch_bounds__(NT, ctas<T, NS, DIM>()) k_f_tvd(const __grid_c
     d0 = d1;
     d1 = dt3;
     fo = R::UP ? ((k + 2) % R::RF) * PL : PL - fo;
-    asm volatile("cp.async.wait_all;\n" ::: "memory");
-    __syncthreads();
+    T* const ct = cur;
+    cur = nxt;
+    nxt = ct;
   }
 }
 
