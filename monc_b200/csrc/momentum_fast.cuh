@@ -168,7 +168,9 @@ __global__ void __launch_bounds__(NT, ctas<T>()) k_f_momentum(const __grid_const
   T u0 = rU[s0 + co], v0 = rV[s0 + co], w0 = rW[s0 + co];
   T pnext = l_thread && kb + 2 <= min(nz, ke + 1) ? level_const(kb + 2) : (T)0.0;
   long long lev = lv0;
-  for (int k = kb; k <= ke; ++k, lev += plane) {
+  const unsigned sa = (unsigned)__cvta_generic_to_shared(rU + sg.soff);
+  long long go = lev + 3 * plane + sg.goff;  // this thread's chunk of level k+3
+  for (int k = kb; k <= ke; ++k, lev += plane, go += plane) {
     T *const t22 = t11 + CN, *const t12 = t22 + CN, *const t13 = t12 + CN, *const t23 = t13 + CN;
     // (loaded a level ahead; level k+1 reads it after this level's barrier)
     if (l_thread && k + 2 <= min(nz, ke + 1)) rL[((k + 2) & (RL - 1)) * L_N + tx] = pnext;
@@ -275,15 +277,16 @@ __global__ void __launch_bounds__(NT, ctas<T>()) k_f_momentum(const __grid_const
     // The stresses of the level are known, no plane of it is read below and level k+2 has landed: one
     // barrier a level.  (A thread ahead writes the next level's stresses to the other buffer.)
     if (k + 3 <= min(nz, ke + 1)) {
-      const long long lv = lev + 3 * plane;
-      sg.copy(rU + s0, d.u + lv);
-      sg.copy(rV + s0, d.v + lv);
-      sg.copy(rW + s0, d.w + lv);
+      const unsigned a = sa + (unsigned)(sizeof(T) * s0);
+      constexpr unsigned RB = sizeof(T) * RP * PL;
+      sg.copy_to(a, d.u + go);
+      sg.copy_to(a + RB, d.v + go);
+      sg.copy_to(a + 2 * RB, d.w + go);
       if (vd) {
-        sg.copy(rZU + s0, d.zu + lv);
-        sg.copy(rZV + s0, d.zv + lv);
-        sg.copy(rZW + s0, d.zw + lv);
-        sg.copy(rVIS + vm_, d.vis + lv);
+        sg.copy_to(a + 3 * RB, d.zu + go);
+        sg.copy_to(a + 4 * RB, d.zv + go);
+        sg.copy_to(a + 5 * RB, d.zw + go);
+        sg.copy_to(sa + 6 * RB + (unsigned)(sizeof(T) * vm_), d.vis + go);
       }
     }
     if (vd) {
@@ -344,7 +347,7 @@ static int launch(const Scalars& s, DevState<T>& d, cudaStream_t st) {
     nsm = n < 1 ? 1 : n;
   }
   const int gx = (s.nx + TX - 1) / TX, gy = (s.ny + TY - 1) / TY, levels = s.nz - 1;
-  const int nc = s.level_chunks > 0 ? s.level_chunks : choose_level_chunks(gx * gy, occ * nsm, levels);
+  const int nc = s.level_chunks > 0 ? s.level_chunks : tvdf::choose_chunks(gx * gy, occ, nsm, levels);
   const int kc = (levels + nc - 1) / nc;
   const dim3 grid(gx, gy, (levels + kc - 1) / kc);
   if (s.tvd_flow) k_f_momentum<T, true><<<grid, NT, smem, st>>>(s, d, kc);

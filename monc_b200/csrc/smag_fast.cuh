@@ -292,7 +292,7 @@ static int launch_as(const Scalars& s, DevState<T>& d, cudaStream_t st) {
     nsm = n < 1 ? 1 : n;
   }
   const int gx = (s.nx + TX - 1) / TX, gy = (s.ny + TY - 1) / TY, levels = s.nz - 2;
-  const int nc = s.level_chunks > 0 ? s.level_chunks : choose_level_chunks(gx * gy, occ * nsm, levels);
+  const int nc = s.level_chunks > 0 ? s.level_chunks : tvdf::choose_chunks(gx * gy, occ, nsm, levels);
   const int kc = (levels + nc - 1) / nc;
   k_f_smag<T, MOIST><<<dim3(gx, gy, 1 + (levels + kc - 1) / kc), NT, smem, st>>>(s, d, kc);
   return 1;

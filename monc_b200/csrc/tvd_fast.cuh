@@ -681,8 +681,25 @@ __global__ void __launch_bounds__(NT, ctas<T, NS, DIM>()) k_f_tvd(const __grid_c
   }
 }
 
-// the number of level chunks: enough CTAs to fill the chip evenly, no chunk shorter than the
-// staging of its first levels is worth
+// The number of chunks the levels are split into.  Where chunks of 8 levels give every resident slot
+// a CTA, choose_level_chunks (256 x 256 x 128 in FP64: theta 0.246 ms at its 8 chunks, 0.243 .. 0.268
+// for 4 .. 16; momentum 0.247, 0.254 .. 0.265).  On smaller grids, where latency counts, shorter
+// chunks: an SM gets m = ceil(tiles n / SMs) CTAs and runs them occ at a time; a CTA takes a level in
+// a time that grows with the CTAs beside it, about as 1 + their number (theta, FP64: 1.3 us alone,
+// 2.0 us for two), and its first levels cost about two more.  64 x 64 x 65 in FP64: 16 chunks, theta
+// 13.7 us (8: 16.2, 22: 18.7, 32: 17.1), subgrid 7.9 (8: 10.4), momentum 12.9 (8: 15.1).
+static inline int choose_chunks(int tiles, int occ, int nsm, int levels) {
+  if ((long long)tiles * (levels / 8) >= (long long)occ * nsm) return choose_level_chunks(tiles, occ * nsm, levels);
+  int best = 1;
+  long long best_cost = -1;
+  for (int n = 1; n <= 64 && 2 * n <= levels; ++n) {
+    const long long m = ((long long)tiles * n + nsm - 1) / nsm, rest = m % occ;
+    const long long cost = ((m / occ) * (occ + 1) + (rest ? rest + 1 : 0)) * ((levels + n - 1) / n + 2);
+    if (best_cost < 0 || cost < best_cost) { best_cost = cost; best = n; }
+  }
+  return best;
+}
+
 template <typename T, int NS, bool CLOUD, int DIM>
 static int launch(const Scalars& s, const Job<T, NS>& job, cudaStream_t st) {
   const size_t smem = smem_bytes<T, NS, DIM>();
@@ -698,7 +715,7 @@ static int launch(const Scalars& s, const Job<T, NS>& job, cudaStream_t st) {
     nsm = n < 1 ? 1 : n;
   }
   const int gx = (s.nx + TX - 1) / TX, gy = (s.ny + TY - 1) / TY, levels = s.nz - 1;
-  const int nc = s.level_chunks > 0 ? s.level_chunks : choose_level_chunks(gx * gy, occ * nsm, levels, 0.002);
+  const int nc = s.level_chunks > 0 ? s.level_chunks : choose_chunks(gx * gy, occ, nsm, levels);
   const int kc = (levels + nc - 1) / nc;
   k_f_tvd<T, NS, CLOUD, DIM><<<dim3(gx, gy, (levels + kc - 1) / kc), NT, smem, st>>>(s, job, kc);
   return 1;
