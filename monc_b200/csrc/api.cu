@@ -766,9 +766,9 @@ static int step_once(mgpu_handle* h, DevState<T>& d) {
                                                  fwd ? nullptr : d.zq_n, h->sc.ugal, h->sc.vgal,
                                                  1.0 - 2.0 * h->sc.tsmth, h->sc.tsmth, h->olbar_d, h->stream);
   }
-  // The FFT solve of a power-of-two nx forms the source inside its first transform (fast
-  // build); the reproducible build keeps the source kernel, whose rounding the oracle matches.
-  const bool src_in_fft = !h->cfg.reproducible && h->cfg.solver == MGPU_SOLVER_FFT && (h->cfg.nx & (h->cfg.nx - 1)) == 0;
+  // The FFT solve forms the source inside its first transform (fast build); the reproducible build
+  // keeps the source kernel, whose rounding the oracle matches.
+  const bool src_in_fft = !h->cfg.reproducible && h->cfg.solver == MGPU_SOLVER_FFT;
   const SourceFields<T> src{d.zu_n, d.zv_n, d.zw_n};
   if (!src_in_fft) {
     if (h->cfg.reproducible) exact::launch_fused_pressure_source<T>(h->sc, d, h->stream);

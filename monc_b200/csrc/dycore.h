@@ -60,8 +60,8 @@ struct SourceFields {
   const T* zw;
 };
 // evs: NULL, or 6 events recorded before, between and after the five kernels.  transpose: apply
-// the transpose of the solve (the adjoint of the pressure solve) instead.  src: when given (and
-// nx is a power of two), the forward x transform forms the pressure source from these fields
+// the transpose of the solve (the adjoint of the pressure solve) instead.  src: when given, the
+// forward x transform forms the pressure source from these fields
 // itself and p's input is not read; the solution is written to p as always.
 template <typename T>
 void fft_solve(const FftPlanDev& plan, const Scalars& s, T* p, cudaStream_t st, int64_t* launches,

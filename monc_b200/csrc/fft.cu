@@ -19,6 +19,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstdio>
+#include <map>
 #include <vector>
 
 #include <mutex>
@@ -441,71 +442,151 @@ __global__ void __launch_bounds__(line_block(LOGN)) k_fft_y(typename Cx<T>::t* _
 // ---- lengths that are not powers of two: mixed-radix Stockham passes in shared memory ---------
 // MONC's FFTPACK factorises any length (cffti1.f90 tries 4, 2, 3, 5, then odd factors); the
 // lengths with prime factors 2, 3 and 5 only (96, 384, 100, 360, ...) take these kernels.  A line
-// of n points sits in shared memory (two buffers, ping-pong) and is transformed by the threads of
-// its block: pass p of radix R (4, 2, 3 or 5) and span NS forms, for j < n/R, the R points
-// x[j + r n/R], multiplies point r by W_{NS R}^{(j mod NS) r} = tw[(j mod NS) r n/(NS R)] (the
-// same table of W_n^q the power-of-two kernels use), applies the R-point DFT and stores point r
-// to y[(j/NS) NS R + j mod NS + r NS] -- the self-sorting form of the radix-16 passes above with
-// the radix varying from pass to pass, so the last pass leaves the result in natural order.
-struct GenFactors {
-  int n, npass;
-  int radix[16];
+// of n points sits in shared memory and is transformed in place: pass p of radix R and span NS
+// gives each of n/R threads the R points x[j + r n/R], which it multiplies by W_{NS R}^{(j mod NS) r} =
+// tw[(j mod NS) r n/(NS R)] (the same table of W_n^q the power-of-two kernels use), transforms by an
+// R-point DFT in registers and stores to y[(j/NS) NS R + j mod NS + r NS] -- the self-sorting form
+// of the radix-16 passes above with the radix varying from pass to pass, so the last pass leaves the
+// result in natural order.
+//
+// Radices go up to 10, composite ones built in registers, so that most lengths take two or three
+// passes (360 = 6 6 10; 12, 15 and 16 would need more registers than two blocks per SM leave; the passes of radix 4, 2, 3 and 5 these replace were five, each with a
+// barrier, a division per point and its own twiddle loads); a block holds as many lines as give its
+// threads one butterfly each.  360 x 300 x 81, FP64: x forward with the pressure source, a kernel of
+// its own before, 0.058 + 0.146 -> 0.115, y 0.190 + 0.176 -> 0.098 + 0.094, x inverse 0.142 -> 0.076 ms
+// (the bytes of a transform take 0.021 ms; some 220 instructions per point at a quarter of the issue
+// slots with 16 warps per SM).  Radices up to 6 without spills: 0.124, 0.115 + 0.109, 0.089.
+struct GenPlan {
+  int n = 0, npass = 0;
+  int lines = 0, block = 0;  // lines per block (a power of two) and threads per block
+  int pitch = 0;             // padded line length, odd
+  int radix[8] = {}, ns[8] = {};
+  unsigned m_nb[8] = {}, m_ns[8] = {};  // ceil(2^32 / (n / radix)), ceil(2^32 / ns): exact quotients below 2^16
+  unsigned m_n = 0, m_h = 0;            // the same for n and n/2 + 1
 };
+constexpr int GEN_RADICES[] = {10, 9, 8, 6, 5, 4, 3, 2};
+constexpr int GEN_BLOCK = 256, GEN_BLOCK_MAX = 1024;
+// threads a block is filled up to with lines: x lines are independent, so small blocks, whose barriers
+// wait for few warps, run best (64: 0.076 ms for the inverse of 360 x 300 x 81, 256: 0.090); a y
+// block's columns make its accesses wide (128: 0.098, 64: 0.105)
+constexpr int GEN_X_THREADS = 64, GEN_Y_THREADS = 128;
+template <typename T, int BLOCK>
+constexpr int gen_ctas() { return BLOCK == GEN_BLOCK_MAX ? 1 : (sizeof(T) == 4 ? 4 : 2); }
 
-// factors of n in the order the passes use them (4s, then 2, 3s, 5s); false if n has another
-// prime factor or is out of range
-static bool gen_factor(int n, GenFactors& g) {
-  g.n = n;
-  g.npass = 0;
-  if (n < 2 || n > 4096) return false;
-  int m = n;
-  while (m % 4 == 0) { g.radix[g.npass++] = 4; m /= 4; }
-  while (m % 2 == 0) { g.radix[g.npass++] = 2; m /= 2; }
-  while (m % 3 == 0) { g.radix[g.npass++] = 3; m /= 3; }
-  while (m % 5 == 0) { g.radix[g.npass++] = 5; m /= 5; }
-  return m == 1 && g.npass <= 16;
+// the passes of the remaining factor m: fewest first, then the largest smallest radix (fewest
+// threads per line), then the smallest largest one
+static void gen_search(int m, int last, int* cur, int np, int* best, int& best_np, int& best_lo, int& best_hi) {
+  if (m == 1) {
+    int lo = 1 << 20, hi = 0;
+    for (int q = 0; q < np; ++q) { lo = std::min(lo, cur[q]); hi = std::max(hi, cur[q]); }
+    if (best_np == 0 || np < best_np || (np == best_np && (lo > best_lo || (lo == best_lo && hi < best_hi)))) {
+      best_np = np; best_lo = lo; best_hi = hi;
+      for (int q = 0; q < np; ++q) best[q] = cur[q];
+    }
+    return;
+  }
+  if (np == 8 || (best_np && np + 1 > best_np)) return;
+  for (int R : GEN_RADICES)
+    if (R <= last && m % R == 0) {
+      cur[np] = R;
+      gen_search(m / R, R, cur, np + 1, best, best_np, best_lo, best_hi);
+    }
 }
 
-// the R-point DFTs; forward uses W_R = e^{-2 pi i / R}, inverse its conjugate.  The constants are
-// cos and sin of 2 pi/3, 2 pi/5 and 4 pi/5 to 30 digits.
-template <typename C>
-__device__ __forceinline__ C cmul_i(C a, bool inv) {  // a * (-i) forward, a * (+i) inverse
+// true if n has no prime factor above 5 and is a length the solve takes
+static bool gen_length(int n) {
+  if (n < 2 || n > 4096) return false;
+  for (int f : {2, 3, 5})
+    while (n % f == 0) n /= f;
+  return n == 1;
+}
+
+// the plan of length n, kept for the lengths seen (at most one per admissible length)
+static bool gen_plan(int n, GenPlan& out, int target) {
+  if (!gen_length(n)) return false;
+  static std::mutex mu;
+  static std::map<std::pair<int, int>, GenPlan> plans;
+  std::lock_guard<std::mutex> lock(mu);
+  auto it = plans.find({n, target});
+  if (it == plans.end()) {
+    GenPlan g;
+    int cur[8], best[8], np = 0, lo = 0, hi = 0;
+    gen_search(n, 10, cur, 0, best, np, lo, hi);
+    if (np == 0) return false;
+    g.n = n;
+    g.npass = np;
+    g.m_n = (unsigned)(((1ull << 32) + n - 1) / n);
+    g.m_h = (unsigned)(((1ull << 32) + n / 2) / (n / 2 + 1));
+    int ns = 1;
+    for (int q = 0; q < np; ++q) {
+      const int R = best[np - 1 - q];  // the smallest radix first, where no twiddles are needed
+      g.radix[q] = R;
+      g.ns[q] = ns;
+      g.m_nb[q] = (unsigned)(((1ull << 32) + n / R - 1) / (n / R));
+      g.m_ns[q] = ns == 1 ? 0u : (unsigned)(((1ull << 32) + ns - 1) / ns);
+      ns *= R;
+    }
+    const int per_line = n / lo;
+    g.lines = 1;
+    while (g.lines < 32 && 2 * g.lines * per_line <= target) g.lines *= 2;
+    g.block = (g.lines * per_line + 31) / 32 * 32;
+    if (g.block > GEN_BLOCK_MAX) return false;
+    g.pitch = (n + n / 8 + 1) | 1;
+    it = plans.emplace(std::make_pair(n, target), g).first;
+  }
+  out = it->second;
+  return true;
+}
+// shared-memory index of point i of a line: one element of padding after every 8, against the
+// strides of the passes' stores
+__device__ __forceinline__ int gpad(int i) { return i + (i >> 3); }
+
+// The R-point DFTs in registers, natural order in and out; forward uses W_R = e^{-2 pi i / R},
+// inverse its conjugate.  The constants are cos and sin of 2 pi/3, 2 pi/5, 4 pi/5 and of 2 pi/9, 4
+// pi/9 and 8 pi/9.
+template <typename C, bool INV>
+__device__ __forceinline__ C cmul_i(C a) {  // a * (-i) forward, a * (+i) inverse
   C r;
-  if (inv) { r.x = -a.y; r.y = a.x; } else { r.x = a.y; r.y = -a.x; }
+  if (INV) { r.x = -a.y; r.y = a.x; } else { r.x = a.y; r.y = -a.x; }
   return r;
 }
 template <typename C, typename T>
 __device__ __forceinline__ C cscale(C a, T s) { C r; r.x = a.x * s; r.y = a.y * s; return r; }
+template <typename C, bool INV, typename T>
+__device__ __forceinline__ C cmul_const(C a, T c, T s) {  // a * (c - i s) forward, a * (c + i s) inverse
+  C r;
+  const T w = INV ? s : -s;
+  r.x = a.x * c - a.y * w;
+  r.y = a.x * w + a.y * c;
+  return r;
+}
 
-template <typename T, typename C>
-__device__ __forceinline__ void gen_dft(C* v, int R, bool inv) {
-  if (R == 2) {
+template <typename T, typename C, int R, bool INV>
+__device__ __forceinline__ void gen_dft(C* v) {
+  if constexpr (R == 2) {
     const C a = v[0], b = v[1];
     v[0] = cadd(a, b);
     v[1] = csub(a, b);
-  } else if (R == 4) {
+  } else if constexpr (R == 4) {
     const C t0 = cadd(v[0], v[2]), t1 = csub(v[0], v[2]), t2 = cadd(v[1], v[3]);
-    const C t3 = cmul_i(csub(v[1], v[3]), inv);
+    const C t3 = cmul_i<C, INV>(csub(v[1], v[3]));
     v[0] = cadd(t0, t2);
     v[2] = csub(t0, t2);
     v[1] = cadd(t1, t3);
     v[3] = csub(t1, t3);
-  } else if (R == 3) {
+  } else if constexpr (R == 3) {
     const T c = (T)-0.5;
-    const T sn = inv ? (T)0.866025403784438646763723170753 : (T)-0.866025403784438646763723170753;
+    const T sn = INV ? (T)0.866025403784438646763723170753 : (T)-0.866025403784438646763723170753;
     const C t1 = cadd(v[1], v[2]);
     const C t2 = cadd(v[0], cscale(t1, c));
     const C d = cscale(csub(v[1], v[2]), sn);  // i * d is added to y1
-    C y1, y2;
-    y1.x = t2.x - d.y; y1.y = t2.y + d.x;
-    y2.x = t2.x + d.y; y2.y = t2.y - d.x;
     v[0] = cadd(v[0], t1);
-    v[1] = y1;
-    v[2] = y2;
-  } else {  // R == 5
+    v[1].x = t2.x - d.y; v[1].y = t2.y + d.x;
+    v[2].x = t2.x + d.y; v[2].y = t2.y - d.x;
+  } else if constexpr (R == 5) {
     const T c1 = (T)0.309016994374947424102293417183, c2 = (T)-0.809016994374947424102293417183;
-    const T s1 = inv ? (T)0.951056516295153572116439333379 : (T)-0.951056516295153572116439333379;
-    const T s2 = inv ? (T)0.587785252292473129180916317273 : (T)-0.587785252292473129180916317273;
+    const T s1 = INV ? (T)0.951056516295153572116439333379 : (T)-0.951056516295153572116439333379;
+    const T s2 = INV ? (T)0.587785252292473129180916317273 : (T)-0.587785252292473129180916317273;
     const C a1 = cadd(v[1], v[4]), a2 = cadd(v[2], v[3]);
     const C b1 = csub(v[1], v[4]), b2 = csub(v[2], v[3]);
     const C x0 = v[0];
@@ -518,79 +599,180 @@ __device__ __forceinline__ void gen_dft(C* v, int R, bool inv) {
     v[4].x = r1.x + q1.y; v[4].y = r1.y - q1.x;
     v[2].x = r2.x - q2.y; v[2].y = r2.y + q2.x;
     v[3].x = r2.x + q2.y; v[3].y = r2.y - q2.x;
-  }
-}
-
-// Transform `nl` lines of n points held at a + l*n (l < nl) in shared memory; b is scratch of the
-// same size.  Returns the buffer holding the result.  All threads of the block take part.
-template <typename T, bool INV>
-__device__ typename Cx<T>::t* gen_lines_fft(typename Cx<T>::t* a, typename Cx<T>::t* b, int nl, const GenFactors& g,
-                                            const typename Cx<T>::t* __restrict__ tw) {
-  typedef typename Cx<T>::t C;
-  const int n = g.n;
-  int ns = 1;
-  for (int p = 0; p < g.npass; ++p) {
-    const int R = g.radix[p], nb = n / R, step = n / (ns * R);
-    for (int t = threadIdx.x; t < nl * nb; t += blockDim.x) {
-      const int l = t / nb, j = t - l * nb;
-      const C* x = a + l * n;
-      C* y = b + l * n;
-      const int jm = j % ns;
-      C v[5];
-      for (int r = 0; r < R; ++r) {
-        C z = x[j + r * nb];
-        if (r > 0 && jm > 0) {
-          C w = tw[jm * r * step];
-          if (INV) w.y = -w.y;
-          z = cmul(z, w);
-        }
-        v[r] = z;
-      }
-      gen_dft<T, C>(v, R, INV);
-      const int o = (j / ns) * ns * R + jm;
-      for (int r = 0; r < R; ++r) y[o + r * ns] = v[r];
+  } else if constexpr (R == 8) {
+    dft_reg<C, R, INV>(v);
+  } else if constexpr (R == 9) {
+    // three 3-point DFTs, twiddles W_9^{ab}, three 3-point DFTs
+    const T c1 = (T)0.766044443118978035202392650555, s1 = (T)0.642787609686539326322643409907;   // 2 pi/9
+    const T c2 = (T)0.173648177666930348851716626769, s2 = (T)0.984807753012208059366743024589;   // 4 pi/9
+    const T c4 = (T)-0.939692620785908384054109277325, s4 = (T)0.342020143325668733044099614682;  // 8 pi/9
+    C u[3][3];
+#pragma unroll
+    for (int b = 0; b < 3; ++b) {
+      C w[3] = {v[b], v[b + 3], v[b + 6]};
+      gen_dft<T, C, 3, INV>(w);
+#pragma unroll
+      for (int a = 0; a < 3; ++a) u[a][b] = w[a];
     }
-    __syncthreads();
-    C* tmp = a; a = b; b = tmp;
-    ns *= R;
+    u[1][1] = cmul_const<C, INV>(u[1][1], c1, s1);
+    u[1][2] = cmul_const<C, INV>(u[1][2], c2, s2);
+    u[2][1] = cmul_const<C, INV>(u[2][1], c2, s2);
+    u[2][2] = cmul_const<C, INV>(u[2][2], c4, s4);
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+      gen_dft<T, C, 3, INV>(u[a]);
+#pragma unroll
+      for (int b = 0; b < 3; ++b) v[a + 3 * b] = u[a][b];
+    }
+  } else {
+    // R = A B with A, B coprime (Good and Thomas): point B a + A b enters at (a, b); W_R^{(B a + A b) k}
+    // = W_A^{a k} W_B^{b k}, so the A- and B-point transforms need no twiddles and give point k at (k mod
+    // A, k mod B)
+    constexpr int A = 2, B = R / A;
+    static_assert(R == 6 || R == 10, "two coprime factors");
+    C u[A][B];
+#pragma unroll
+    for (int a = 0; a < A; ++a) {
+#pragma unroll
+      for (int b = 0; b < B; ++b) u[a][b] = v[(B * a + A * b) % R];
+      gen_dft<T, C, B, INV>(u[a]);
+    }
+#pragma unroll
+    for (int kb = 0; kb < B; ++kb) {
+      C w[A];
+#pragma unroll
+      for (int a = 0; a < A; ++a) w[a] = u[a][kb];
+      gen_dft<T, C, A, INV>(w);
+#pragma unroll
+      for (int ka = 0; ka < A; ++ka)
+#pragma unroll
+        for (int k = 0; k < R; ++k)
+          if (k % A == ka && k % B == kb) v[k] = w[ka];
+    }
   }
-  return a;
 }
 
-constexpr int GEN_BLOCK = 128;
-
-// forward x of generic length: one block per row pair, packed, transformed and split as
-// k_fft_x_fwd does it
-template <typename T>
-__global__ void __launch_bounds__(GEN_BLOCK) k_fftg_x_fwd(const T* __restrict__ p, typename Cx<T>::t* __restrict__ spec,
-                                                          const typename Cx<T>::t* __restrict__ tw, GenFactors g, int ny,
-                                                          int nz, int p_rows, int p_row0, int nblk) {
+// one pass of radix R over nl lines (at a + l * pitch), in place; every thread of the block calls it
+template <typename T, int R, bool INV>
+__device__ __forceinline__ void gen_pass(typename Cx<T>::t* a, int pitch, int nl, int n, int ns, unsigned m_nb,
+                                         unsigned m_ns, const typename Cx<T>::t* __restrict__ tw) {
   typedef typename Cx<T>::t C;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int n = g.n, nxh = n / 2 + 1, pairs = ny / 2;
-  C* a = reinterpret_cast<C*>(smem_raw);
-  C* b = a + n;
-  const int pr = blockIdx.x;
-  const int k = pr / pairs + 1, jr = 2 * (pr % pairs);
-  const T* row = p + ((long long)(k - 1) * p_rows + p_row0 + jr) * n;
-  for (int e = threadIdx.x; e < n; e += blockDim.x) {
-    C z;
-    z.x = row[e];
-    z.y = row[n + e];
-    a[e] = z;
+  const int nb = n / R, t = threadIdx.x;
+  const bool on = t < nl * nb;
+  const int l = nb == 1 ? t : (int)__umulhi((unsigned)t, m_nb), j = t - l * nb;
+  const int q = ns == 1 ? j : (int)__umulhi((unsigned)j, m_ns), jm = j - q * ns;
+  C* x = a + l * pitch;
+  C v[R];
+  if (on) {
+#pragma unroll
+    for (int r = 0; r < R; ++r) v[r] = x[gpad(j + r * nb)];
+    if (ns > 1) {
+      const int step = jm * (nb / ns);
+#pragma unroll
+      for (int r = 1; r < R; ++r) v[r] = mul_tw<C, INV>(v[r], __ldg(tw + r * step));
+    }
+    gen_dft<T, C, R, INV>(v);
   }
   __syncthreads();
-  const C* zt = gen_lines_fft<T, false>(a, b, 1, g, tw);
-  for (int m = threadIdx.x; m < nxh; m += blockDim.x) {
-    const C zm = zt[m];
-    const C zn = zt[(n - m) % n];
+  if (on) {
+    const int o = q * ns * R + jm;
+#pragma unroll
+    for (int r = 0; r < R; ++r) x[gpad(o + r * ns)] = v[r];
+  }
+  __syncthreads();
+}
+
+template <typename T, bool INV>
+__device__ __forceinline__ void gen_lines_fft(typename Cx<T>::t* a, int nl, const GenPlan& g,
+                                              const typename Cx<T>::t* __restrict__ tw) {
+  for (int p = 0; p < g.npass; ++p) {
+#define MGPU_GEN_PASS(R) \
+  case R: gen_pass<T, R, INV>(a, g.pitch, nl, g.n, g.ns[p], g.m_nb[p], g.m_ns[p], tw); break;
+    switch (g.radix[p]) {
+      MGPU_GEN_PASS(2) MGPU_GEN_PASS(3) MGPU_GEN_PASS(4) MGPU_GEN_PASS(5) MGPU_GEN_PASS(6) MGPU_GEN_PASS(8) MGPU_GEN_PASS(9) MGPU_GEN_PASS(10)
+
+    }
+#undef MGPU_GEN_PASS
+  }
+}
+
+// a block's row pairs: level and first row of each, and what the pressure source takes from them
+template <typename T>
+struct GenLine {
+  int k, jr;
+  long long row;  // offset of row jr in a field of p_rows rows per level
+  long long vm;   // offset of the row below it, periodic
+  T tzc1, tzc2;
+};
+
+// forward x of generic length: a block's row pairs, packed, transformed and split as k_fft_x_fwd does
+// it; with SRC the pressure source is formed from the stepped velocities (see k_fft_x_fwd_src; one
+// domain, all rows)
+template <typename T, int BLOCK, bool SRC>
+__global__ void __launch_bounds__(BLOCK, gen_ctas<T, BLOCK>()) k_fftg_x_fwd(const T* __restrict__ p, typename Cx<T>::t* __restrict__ spec,
+                                                      const typename Cx<T>::t* __restrict__ tw, GenPlan g, int ny, int nz,
+                                                      int p_rows, int p_row0, int nblk, Scalars s, SourceFields<T> f) {
+  typedef typename Cx<T>::t C;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ GenLine<T> li[32];
+  const int n = g.n, nxh = n / 2 + 1, pairs = ny / 2;
+  C* a = reinterpret_cast<C*>(smem_raw);
+  const int pr0 = blockIdx.x * g.lines, nl = min(g.lines, nz * pairs - pr0);
+  if ((int)threadIdx.x < nl) {
+    GenLine<T>& q = li[threadIdx.x];
+    const int pr = pr0 + threadIdx.x;
+    q.k = pr / pairs + 1;
+    q.jr = 2 * (pr % pairs);
+    const long long lv = (long long)(q.k - 1) * p_rows + p_row0;
+    q.row = (lv + q.jr) * n;
+    q.vm = (lv + (q.jr == 0 ? ny - 1 : q.jr - 1)) * n;
+    if constexpr (SRC) {
+      q.tzc1 = (T)__ldg(s.prof + P_TZC1 * (nz + 2) + q.k);
+      q.tzc2 = (T)__ldg(s.prof + P_TZC2 * (nz + 2) + q.k);
+    }
+  }
+  __syncthreads();
+  const T timec = s.forward ? (T)(1.0 / s.dtm) : (T)(1.0 / (2.0 * s.dtm)), cx = (T)s.cx, cy = (T)s.cy;
+#pragma unroll 4
+  for (int t = threadIdx.x; t < nl * n; t += blockDim.x) {
+    const int l = (int)__umulhi((unsigned)t, g.m_n), e = t - l * n;
+    const GenLine<T>& q = li[l];
+    C z;
+    if constexpr (SRC) {
+      auto one = [&](long long r, long long rm) {
+        const int em = e == 0 ? n - 1 : e - 1;
+        T pp = (T)0.0;
+        pp = pp + cx * (__ldg(f.zu + r + e) - __ldg(f.zu + r + em));
+        pp = pp + cy * (__ldg(f.zv + r + e) - __ldg(f.zv + rm + e));
+        pp = pp + (T)4.0 * (q.tzc2 * __ldg(f.zw + r + e) - q.tzc1 * __ldg(f.zw + r - s.plane + e));
+        return pp * timec;
+      };
+      z.x = z.y = (T)0;
+      if (q.k > 1) {
+        z.x = one(q.row, q.vm);
+        z.y = one(q.row + n, q.row);
+      }
+    } else {
+      z.x = p[q.row + e];
+      z.y = p[q.row + n + e];
+    }
+    a[l * g.pitch + gpad(e)] = z;
+  }
+  __syncthreads();
+  gen_lines_fft<T, false>(a, nl, g, tw);
+#pragma unroll 2
+  for (int t = threadIdx.x; t < nl * nxh; t += blockDim.x) {
+    const int l = (int)__umulhi((unsigned)t, g.m_h), m = t - l * nxh;
+    const C* zt = a + l * g.pitch;
+    const C zm = zt[gpad(m)];
+    const C zn = zt[gpad(m == 0 ? 0 : n - m)];
     C ra, rb;
     ra.x = (T)0.5 * (zm.x + zn.x);
     ra.y = (T)0.5 * (zm.y - zn.y);
     rb.x = (T)0.5 * (zm.y + zn.y);
     rb.y = (T)0.5 * (zn.x - zm.x);
     int w;
-    C* o = spec + spec_x_offset(m, nxh, nblk, ny, nz, k, jr, &w);
+    C* o = spec + spec_x_offset(m, nxh, nblk, ny, nz, li[l].k, li[l].jr, &w);
     o[0] = ra;
     o[w] = rb;
   }
@@ -598,76 +780,107 @@ __global__ void __launch_bounds__(GEN_BLOCK) k_fftg_x_fwd(const T* __restrict__ 
 
 // inverse x of generic length, the inverse of k_fftg_x_fwd (imaginary parts of kx = 0 and, for
 // even n, kx = n/2 dropped)
-template <typename T>
-__global__ void __launch_bounds__(GEN_BLOCK) k_fftg_x_inv(T* __restrict__ p, const typename Cx<T>::t* __restrict__ spec,
-                                                          const typename Cx<T>::t* __restrict__ tw, GenFactors g, int ny,
-                                                          int nz, int p_rows, int p_row0, int nblk) {
+template <typename T, int BLOCK>
+__global__ void __launch_bounds__(BLOCK, gen_ctas<T, BLOCK>()) k_fftg_x_inv(T* __restrict__ p, const typename Cx<T>::t* __restrict__ spec,
+                                                      const typename Cx<T>::t* __restrict__ tw, GenPlan g, int ny, int nz,
+                                                      int p_rows, int p_row0, int nblk) {
   typedef typename Cx<T>::t C;
   extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ GenLine<T> li[32];
   const int n = g.n, nxh = n / 2 + 1, pairs = ny / 2;
   C* a = reinterpret_cast<C*>(smem_raw);
-  C* b = a + n;
-  const int pr = blockIdx.x;
-  const int k = pr / pairs + 1, jr = 2 * (pr % pairs);
-  for (int m = threadIdx.x; m < nxh; m += blockDim.x) {
+  const int pr0 = blockIdx.x * g.lines, nl = min(g.lines, nz * pairs - pr0);
+  if ((int)threadIdx.x < nl) {
+    GenLine<T>& q = li[threadIdx.x];
+    const int pr = pr0 + threadIdx.x;
+    q.k = pr / pairs + 1;
+    q.jr = 2 * (pr % pairs);
+    q.row = ((long long)(q.k - 1) * p_rows + p_row0 + q.jr) * n;
+  }
+  __syncthreads();
+#pragma unroll 4
+  for (int t = threadIdx.x; t < nl * nxh; t += blockDim.x) {
+    const int l = (int)__umulhi((unsigned)t, g.m_h), m = t - l * nxh;
+    C* x = a + l * g.pitch;
     int w;
-    const C* in = spec + spec_x_offset(m, nxh, nblk, ny, nz, k, jr, &w);
+    const C* in = spec + spec_x_offset(m, nxh, nblk, ny, nz, li[l].k, li[l].jr, &w);
     C ra = in[0], rb = in[w];
     const bool nyquist = 2 * m == n;
     if (m == 0 || nyquist) { ra.y = (T)0; rb.y = (T)0; }
     C z;
     z.x = ra.x - rb.y;
     z.y = ra.y + rb.x;
-    a[m] = z;
+    x[gpad(m)] = z;
     if (m > 0 && !nyquist) {
       C zc;
       zc.x = ra.x + rb.y;
       zc.y = rb.x - ra.y;
-      a[n - m] = zc;
+      x[gpad(n - m)] = zc;
     }
   }
   __syncthreads();
-  const C* zt = gen_lines_fft<T, true>(a, b, 1, g, tw);
-  T* row = p + ((long long)(k - 1) * p_rows + p_row0 + jr) * n;
+  gen_lines_fft<T, true>(a, nl, g, tw);
   const T sc = (T)(1.0 / (double)n);
-  for (int e = threadIdx.x; e < n; e += blockDim.x) {
-    row[e] = zt[e].x * sc;
-    row[n + e] = zt[e].y * sc;
+#pragma unroll 4
+  for (int t = threadIdx.x; t < nl * n; t += blockDim.x) {
+    const int l = (int)__umulhi((unsigned)t, g.m_n), e = t - l * n;
+    const C z = a[l * g.pitch + gpad(e)];
+    p[li[l].row + e] = z.x * sc;
+    p[li[l].row + n + e] = z.y * sc;
   }
 }
 
-// columns per block of the generic y kernel: as many as keep the two buffers within 64 KB of
-// FP64 lines (at least one)
-static int gen_y_cols(int n) { return std::max(1, std::min(8, 2048 / n)); }
-
-// y of generic length on a tile of kx columns of one level, the layout of k_fft_y; the inverse
-// is scaled by 1/n
-template <typename T, bool INV>
-__global__ void __launch_bounds__(GEN_BLOCK) k_fftg_y(typename Cx<T>::t* __restrict__ spec,
-                                                      const typename Cx<T>::t* __restrict__ tw, GenFactors g, int ncols,
-                                                      int nz, int rpb, int tc) {
+// y of generic length on a tile of g.lines kx columns of one level, the layout of k_fft_y; the
+// inverse is scaled by 1/n
+template <typename T, int BLOCK, bool INV>
+__global__ void __launch_bounds__(BLOCK, gen_ctas<T, BLOCK>()) k_fftg_y(typename Cx<T>::t* __restrict__ spec,
+                                                  const typename Cx<T>::t* __restrict__ tw, GenPlan g, int ncols, int nz,
+                                                  int rpb) {
   typedef typename Cx<T>::t C;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int n = g.n;
+  const int n = g.n, lg = __ffs(g.lines) - 1;
   C* a = reinterpret_cast<C*>(smem_raw);
-  C* b = a + (size_t)tc * n;
-  const int kx0 = blockIdx.x * tc, k = blockIdx.y + 1;
-  const int nc = min(tc, ncols - kx0);
-  for (int t = threadIdx.x; t < nc * n; t += blockDim.x) {
-    const int e = t / nc, c = t - e * nc;  // consecutive threads take consecutive columns
-    a[c * n + e] = spec[spec_row(e, k, rpb, ncols, nz) + kx0 + c];
-  }
+  const int kx0 = blockIdx.x << lg, k = blockIdx.y + 1;
+  const int nc = min(g.lines, ncols - kx0);
+  // consecutive threads take consecutive columns
+  const int c = threadIdx.x & (g.lines - 1), e0 = threadIdx.x >> lg, de = blockDim.x >> lg;
+  C* x = a + c * g.pitch;
+  C* col = spec + kx0 + c;
+  // (in batches whose loads are in flight together: the shared-memory stores may alias them as far as
+  // the compiler knows)
+  if (c < nc)
+    for (int eb = e0; eb < n; eb += 8 * de) {
+      C z[8];
+#pragma unroll
+      for (int q = 0; q < 8; ++q)
+        if (eb + q * de < n) z[q] = col[spec_row(eb + q * de, k, rpb, ncols, nz)];
+#pragma unroll
+      for (int q = 0; q < 8; ++q)
+        if (eb + q * de < n) x[gpad(eb + q * de)] = z[q];
+    }
   __syncthreads();
-  const C* zt = gen_lines_fft<T, INV>(a, b, nc, g, tw);
+  gen_lines_fft<T, INV>(a, nc, g, tw);
   const T sc = INV ? (T)(1.0 / (double)n) : (T)1.0;
-  for (int t = threadIdx.x; t < nc * n; t += blockDim.x) {
-    const int e = t / nc, c = t - e * nc;
-    C z = zt[c * n + e];
-    if (INV) { z.x = z.x * sc; z.y = z.y * sc; }
-    spec[spec_row(e, k, rpb, ncols, nz) + kx0 + c] = z;
-  }
+  if (c < nc)
+    for (int e = e0; e < n; e += de) {
+      C z = x[gpad(e)];
+      if (INV) { z.x = z.x * sc; z.y = z.y * sc; }
+      col[spec_row(e, k, rpb, ncols, nz)] = z;
+    }
 }
 
+template <typename T>
+static size_t gen_smem(const GenPlan& g) { return (size_t)g.lines * g.pitch * sizeof(typename Cx<T>::t); }
+
+template <typename T, int BLOCK>
+static void gen_attr_of() {
+  const int mx = (int)((4096 + 512 + 128) * sizeof(typename Cx<T>::t));
+  cudaFuncSetAttribute(k_fftg_x_fwd<T, BLOCK, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx);
+  cudaFuncSetAttribute(k_fftg_x_fwd<T, BLOCK, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx);
+  cudaFuncSetAttribute(k_fftg_x_inv<T, BLOCK>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx);
+  cudaFuncSetAttribute(k_fftg_y<T, BLOCK, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx);
+  cudaFuncSetAttribute(k_fftg_y<T, BLOCK, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx);
+}
 template <typename T>
 static void ensure_gen_attr() {
   static std::mutex mu;
@@ -676,11 +889,8 @@ static void ensure_gen_attr() {
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return;
   std::lock_guard<std::mutex> lock(mu);
   if (done[dev]) return;
-  const int mx = (int)(2 * 4096 * sizeof(typename Cx<T>::t));
-  cudaFuncSetAttribute(k_fftg_x_fwd<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx);
-  cudaFuncSetAttribute(k_fftg_x_inv<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx);
-  cudaFuncSetAttribute(k_fftg_y<T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx);
-  cudaFuncSetAttribute(k_fftg_y<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx);
+  gen_attr_of<T, GEN_BLOCK>();
+  gen_attr_of<T, GEN_BLOCK_MAX>();
   done[dev] = true;
 }
 
@@ -720,13 +930,20 @@ template <typename T>
 static void launch_fft_x(bool inverse, int n, T* p, typename Cx<T>::t* spec, const typename Cx<T>::t* tw, int ny,
                          int nz, int p_rows, int p_row0, int nblk, cudaStream_t st) {
   if (!is_pow2(n)) {
-    GenFactors g;
-    if (!gen_factor(n, g)) return;
+    GenPlan g;
+    if (!gen_plan(n, g, GEN_X_THREADS)) return;
     ensure_gen_attr<T>();
-    const unsigned grid = (unsigned)((long long)nz * (ny / 2));
-    const size_t smem = 2 * (size_t)n * sizeof(typename Cx<T>::t);
-    if (inverse) k_fftg_x_inv<T><<<grid, GEN_BLOCK, smem, st>>>(p, spec, tw, g, ny, nz, p_rows, p_row0, nblk);
-    else k_fftg_x_fwd<T><<<grid, GEN_BLOCK, smem, st>>>(p, spec, tw, g, ny, nz, p_rows, p_row0, nblk);
+    const unsigned grid = (unsigned)(((long long)nz * (ny / 2) + g.lines - 1) / g.lines);
+    const size_t smem = gen_smem<T>(g);
+    const Scalars s0{};
+    const SourceFields<T> f0{};
+    if (g.block <= GEN_BLOCK) {
+      if (inverse) k_fftg_x_inv<T, GEN_BLOCK><<<grid, g.block, smem, st>>>(p, spec, tw, g, ny, nz, p_rows, p_row0, nblk);
+      else k_fftg_x_fwd<T, GEN_BLOCK, false><<<grid, g.block, smem, st>>>(p, spec, tw, g, ny, nz, p_rows, p_row0, nblk, s0, f0);
+    } else {
+      if (inverse) k_fftg_x_inv<T, GEN_BLOCK_MAX><<<grid, g.block, smem, st>>>(p, spec, tw, g, ny, nz, p_rows, p_row0, nblk);
+      else k_fftg_x_fwd<T, GEN_BLOCK_MAX, false><<<grid, g.block, smem, st>>>(p, spec, tw, g, ny, nz, p_rows, p_row0, nblk, s0, f0);
+    }
     return;
   }
   const int logn = ilog2(n);
@@ -748,10 +965,21 @@ static void launch_fft_x(bool inverse, int n, T* p, typename Cx<T>::t* spec, con
   }
 }
 
-// forward x-FFT of the pressure source formed from zu, zv, zw (power-of-two nx, one domain)
+// forward x-FFT of the pressure source formed from zu, zv, zw (one domain)
 template <typename T>
 static void launch_fft_x_src(const Scalars& s, const SourceFields<T>& f, typename Cx<T>::t* spec,
                              const typename Cx<T>::t* tw, cudaStream_t st) {
+  if (!is_pow2(s.nx)) {
+    GenPlan g;
+    if (!gen_plan(s.nx, g, GEN_X_THREADS)) return;
+    ensure_gen_attr<T>();
+    const unsigned grid = (unsigned)(((long long)s.nz * (s.ny / 2) + g.lines - 1) / g.lines);
+    if (g.block <= GEN_BLOCK)
+      k_fftg_x_fwd<T, GEN_BLOCK, true><<<grid, g.block, gen_smem<T>(g), st>>>(nullptr, spec, tw, g, s.ny, s.nz, s.ny, 0, 1, s, f);
+    else
+      k_fftg_x_fwd<T, GEN_BLOCK_MAX, true><<<grid, g.block, gen_smem<T>(g), st>>>(nullptr, spec, tw, g, s.ny, s.nz, s.ny, 0, 1, s, f);
+    return;
+  }
   const int logn = ilog2(s.nx);
   ensure_line_attr<T>();
   const long long pairs = (long long)s.nz * (s.ny / 2);
@@ -775,14 +1003,18 @@ template <typename T>
 static void launch_fft_y(bool inverse, int n, typename Cx<T>::t* spec, const typename Cx<T>::t* tw, int ncols, int nz,
                          int rpb, cudaStream_t st) {
   if (!is_pow2(n)) {
-    GenFactors g;
-    if (!gen_factor(n, g)) return;
+    GenPlan g;
+    if (!gen_plan(n, g, GEN_Y_THREADS)) return;
     ensure_gen_attr<T>();
-    const int tc = gen_y_cols(n);
-    dim3 grid((unsigned)((ncols + tc - 1) / tc), (unsigned)nz);
-    const size_t smem = 2 * (size_t)tc * n * sizeof(typename Cx<T>::t);
-    if (inverse) k_fftg_y<T, true><<<grid, GEN_BLOCK, smem, st>>>(spec, tw, g, ncols, nz, rpb, tc);
-    else k_fftg_y<T, false><<<grid, GEN_BLOCK, smem, st>>>(spec, tw, g, ncols, nz, rpb, tc);
+    dim3 grid((unsigned)((ncols + g.lines - 1) / g.lines), (unsigned)nz);
+    const size_t smem = gen_smem<T>(g);
+    if (g.block <= GEN_BLOCK) {
+      if (inverse) k_fftg_y<T, GEN_BLOCK, true><<<grid, g.block, smem, st>>>(spec, tw, g, ncols, nz, rpb);
+      else k_fftg_y<T, GEN_BLOCK, false><<<grid, g.block, smem, st>>>(spec, tw, g, ncols, nz, rpb);
+    } else {
+      if (inverse) k_fftg_y<T, GEN_BLOCK_MAX, true><<<grid, g.block, smem, st>>>(spec, tw, g, ncols, nz, rpb);
+      else k_fftg_y<T, GEN_BLOCK_MAX, false><<<grid, g.block, smem, st>>>(spec, tw, g, ncols, nz, rpb);
+    }
     return;
   }
   const int logn = ilog2(n);
@@ -1104,10 +1336,7 @@ static int plan_tables(FftPlanDev& pl, const RefState& rs) {
 }
 
 // Horizontal transform lengths the solve supports: 4 .. 4096 points with prime factors 2, 3, 5
-bool fft_length_ok(int n) {
-  GenFactors g;
-  return n >= 4 && gen_factor(n, g);
-}
+bool fft_length_ok(int n) { return n >= 4 && gen_length(n); }
 
 int fft_plan_create(FftPlanDev& pl, const Scalars& s, const RefState& rs, bool fp32) {
   pl.nx = s.nx;
@@ -1157,7 +1386,7 @@ void fft_solve(const FftPlanDev& pl, const Scalars& s, T* p, cudaStream_t st, in
   double2* s1 = pl.s1;
   auto mark = [&](int q) { if (evs) cudaEventRecord(evs[q], st); };
   mark(0);
-  if (src && is_pow2(s.nx)) launch_fft_x_src<T>(s, *src, spec, twx, st);
+  if (src) launch_fft_x_src<T>(s, *src, spec, twx, st);
   else launch_fft_x<T>(false, logx, p, spec, twx, s.ny, s.nz, s.ny, 0, 1, st);
   mark(1);
   launch_fft_y<T>(false, logy, spec, twy, pl.nxh, s.nz, s.ny, st);

@@ -73,3 +73,25 @@ def test_transposed_solve_on_generic_grid_is_the_adjoint(gpu_lib):
     m.close()
     lhs, rhs = float(np.vdot(ax, y)), float(np.vdot(x, aty))
     assert abs(lhs - rhs) <= 1e-10 * max(abs(lhs), 1e-300)
+
+
+@pytest.mark.parametrize("precision", [cf.FP64, cf.FP32_MIXED], ids=["fp64", "fp32"])
+@pytest.mark.parametrize("nx,ny,nz", [(6, 10, 5), (18, 250, 5), (486, 12, 5), (1500, 6, 4), (3888, 4, 4), (4, 4050, 4),
+                                      (90, 3750, 4), (30, 14 * 5 - 6, 7)])
+def test_every_kind_of_plan_matches_oracle(gpu_lib, nx, ny, nz, precision):
+    """One pass to five, every radix, one line per block and many, blocks of more than 256 threads; the
+    tolerances are those of the solves above (a transform's error grows with log n only)."""
+    cfg = cf.dry_cbl_config(nx, ny, nz, 50.0, 25.0, 1.0, precision=precision)
+    o, m = po.Oracle(cfg), api.Model(cfg)
+    p = ini.uniform_noise((nz, ny, nx), 9, 8, 1.0)
+    p[0] = 0.0
+    o.set(api.FIELDS["p"], p)
+    m.upload("p", p)
+    o.set_timestep(2)
+    m.set_timestep(2)
+    o.component(api.COMPONENTS["fftsolver"])
+    m.component("fftsolver")
+    e = rel_err(m.download("p"), o.get(api.FIELDS["p"]))
+    assert e <= (1e-11 if precision == cf.FP64 else 2e-4), f"rel err {e:.3e}"
+    m.close()
+    o.close()
