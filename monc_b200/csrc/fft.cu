@@ -1087,54 +1087,61 @@ __device__ __forceinline__ unsigned char* tri_smem() {
 }
 
 // ---- vertical tridiagonal per (ky, kx) in FP64 ----------------------------------------------
-// The horizontal-mean mode (kx = ky = 0) of one column, held at col[0], col[1], ... (level k at
-// col[k-1]): p(1) = p(2) = 0 and an upward recurrence, or with transpose the transposed recurrence
-// from the top.
+// The horizontal-mean mode (kx = ky = 0), by a whole block: p(1) = p(2) = 0 and an upward recurrence
+// over the rows r = 2..nz-1 of cza(r) p(r+1) + czg(r) p(r) + czb(r) p(r-1) = b(r), or with transpose the
+// transposed recurrence from the top.  The column (level k at sp[(k-1) lstride]) is loaded by all
+// threads, which also divide every row by its leading coefficient, so that the one thread that runs the
+// recurrence waits for a multiply-add per level: with the divisions in the recurrence and its operands
+// loaded in turn, this block was the last to finish and set the time of the whole solve (21 of 21 us at
+// 64 x 64 x 65, 31 at 128 x 128 x 96, 41 of 46 at 256 x 256 x 128, FP64).  smem: mean_smem(nz) bytes.
+__host__ __device__ constexpr size_t mean_smem(int nz) { return (size_t)(nz + 2) * (sizeof(double2) + 2 * sizeof(double)); }
 template <typename T>
-__device__ void mean_mode_column(typename Cx<T>::t* col, int nz, const double* czb, const double* cza,
-                                 const double* czg, int transpose) {
+__device__ void mean_mode_block(typename Cx<T>::t* sp, long long lstride, int nz, const double* __restrict__ prof,
+                                int prof_stride, int transpose, unsigned char* smem) {
   typedef typename Cx<T>::t C;
-  C zero;
-  zero.x = (T)0;
-  zero.y = (T)0;
-  if (transpose) {
-    // the rows r = 2..nz-1 of cza(r) p(r+1) + czg(r) p(r) + czb(r) p(r-1) = b(r), p(1) = p(2) = 0,
-    // transposed and solved from the top
-    double zr1 = 0.0, zi1 = 0.0, zr2 = 0.0, zi2 = 0.0;  // z(u), z(u+1)
-    C ynext = col[nz - 1];                              // y(nz)
-    for (int u = nz; u >= 3; --u) {
-      const C yu = ynext;
-      if (u >= 4) ynext = col[u - 2];  // y(u-1), read before z(u-1) overwrites it
-      double yr = (double)yu.x, yi = (double)yu.y;
-      if (u <= nz - 1) { yr -= czg[u] * zr1; yi -= czg[u] * zi1; }
-      if (u + 1 <= nz - 1) { yr -= czb[u + 1] * zr2; yi -= czb[u + 1] * zi2; }
-      const double zr = yr / cza[u - 1], zi = yi / cza[u - 1];  // z(u-1)
-      zr2 = zr1; zi2 = zi1; zr1 = zr; zi1 = zi;
-      C o;
-      o.x = (T)zr;
-      o.y = (T)zi;
-      col[u - 2] = o;
+  double2* bb = reinterpret_cast<double2*>(smem);  // right-hand sides, then the solution
+  double* a1 = reinterpret_cast<double*>(bb + nz + 2);
+  double* a2 = a1 + nz + 2;
+  const double* __restrict__ czb = prof + P_CZB * prof_stride;
+  const double* __restrict__ cza = prof + P_CZA * prof_stride;
+  const double* __restrict__ czg = prof + P_CZG * prof_stride;
+  for (int k = 3 + (int)threadIdx.x; k <= nz; k += blockDim.x) {
+    // step k: p(k) from row k-1 and the two levels below; transposed: z(k-1) from y(k) and the two above
+    const C v = transpose ? sp[(long long)(k - 1) * lstride] : sp[(long long)(k - 2) * lstride];
+    const double r = 1.0 / cza[k - 1];
+    bb[k] = make_double2((double)v.x * r, (double)v.y * r);
+    if (transpose) {
+      a1[k] = k <= nz - 1 ? czg[k] * r : 0.0;
+      a2[k] = k + 1 <= nz - 1 ? czb[k + 1] * r : 0.0;
+    } else {
+      a1[k] = czg[k - 1] * r;
+      a2[k] = czb[k - 1] * r;
     }
-    col[0] = zero;
-    col[nz - 1] = zero;
-    return;
   }
-  C v2 = col[1];
-  double sr_prev = (double)v2.x, si_prev = (double)v2.y;
-  double pr2 = 0.0, pi2 = 0.0, pr1 = 0.0, pi1 = 0.0;  // p(k-2), p(k-1)
-  col[0] = zero;  // p(1) = p(2) = 0 for the mean mode
-  col[1] = zero;
-  for (int k = 3; k <= nz; ++k) {
-    C vk = col[k - 1];
-    double pr = (sr_prev - czg[k - 1] * pr1 - czb[k - 1] * pr2) / cza[k - 1];
-    double pi = (si_prev - czg[k - 1] * pi1 - czb[k - 1] * pi2) / cza[k - 1];
-    sr_prev = (double)vk.x;
-    si_prev = (double)vk.y;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double r1 = 0.0, i1 = 0.0, r2 = 0.0, i2 = 0.0;  // the last two values
+    const int n = nz - 2;
+#pragma unroll 8
+    for (int q = 0; q < n; ++q) {
+      const int k = transpose ? nz - q : 3 + q;
+      const double2 b = bb[k];
+      const double c1 = a1[k], c2 = a2[k];
+      const double r = (b.x - c2 * r2) - c1 * r1, i = (b.y - c2 * i2) - c1 * i1;
+      r2 = r1; i2 = i1; r1 = r; i1 = i;
+      bb[k] = make_double2(r, i);
+    }
+  }
+  __syncthreads();
+  for (int k = 1 + (int)threadIdx.x; k <= nz; k += blockDim.x) {
     C o;
-    o.x = (T)pr;
-    o.y = (T)pi;
-    col[k - 1] = o;
-    pr2 = pr1; pi2 = pi1; pr1 = pr; pi1 = pi;
+    o.x = o.y = (T)0;
+    const int q = transpose ? k + 1 : k;  // the step that gave level k
+    if (q >= 3 && q <= nz) {
+      o.x = (T)bb[q].x;
+      o.y = (T)bb[q].y;
+    }
+    sp[(long long)(k - 1) * lstride] = o;
   }
 }
 
@@ -1161,14 +1168,7 @@ __global__ void k_tridiag(typename Cx<T>::t* __restrict__ spec, double2* __restr
   const double* cza = cf + cs;
   const double* czg = cf + 2 * cs;
   if (kx0 == 0 && blockIdx.x == gridDim.x - 1) {
-    // the mean mode is one sequential recurrence over the levels: stage its column (row 0,
-    // column 0 of every level) in shared memory so that no step of it waits on a global load
-    C* colv = reinterpret_cast<C*>(tri_smem());
-    for (int k = threadIdx.x; k < nz; k += blockDim.x) colv[k] = spec[(long long)k * lstride];
-    __syncthreads();
-    if (threadIdx.x == 0) mean_mode_column<T>(colv, nz, czb, cza, czg, transpose);
-    __syncthreads();
-    for (int k = threadIdx.x; k < nz; k += blockDim.x) spec[(long long)k * lstride] = colv[k];
+    mean_mode_block<T>(spec, lstride, nz, prof, prof_stride, transpose, tri_smem());  // row 0, column 0 of every level
     return;
   }
   long long col = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -1280,12 +1280,153 @@ __global__ void k_tridiag(typename Cx<T>::t* __restrict__ spec, double2* __restr
   cp_async_wait_0();
 }
 
+// The same solve for grids with few columns, where one thread per column leaves most of the chip idle
+// and the two sweeps' latency is the time: the levels 2 .. nz of a column are cut into segments of LV
+// levels, one thread each, held in registers.  Each recurrence is linear in the value that enters
+// the segment, so a segment first forms its end value for zero and the factor that value enters with,
+// the threads chain those through shared memory, and every thread runs its levels with the right start.
+// A block is 32 columns (one warp per segment) of up to SEG_MAX segments; as in k_tridiag one extra
+// block takes the mean mode.
+constexpr int SEG_COLS = 32, SEG_MAX = 16;
+template <typename T, int LV>
+__global__ void __launch_bounds__(SEG_COLS * SEG_MAX) k_tridiag_seg(typename Cx<T>::t* __restrict__ spec,
+                                                                   const double* __restrict__ b1,
+                                                                   const double* __restrict__ prof, int prof_stride, int nx,
+                                                                   int ny, int nz, int transpose, int ncols, int kx0, int rpb) {
+  typedef typename Cx<T>::t C;
+  const int nxh = nx / 2 + 1;
+  const long long lstride = (long long)rpb * ncols;  // level stride of the spectrum
+  const double* __restrict__ czb = prof + P_CZB * prof_stride;
+  const double* __restrict__ cza = prof + P_CZA * prof_stride;
+  if (kx0 == 0 && blockIdx.x == gridDim.x - 1) {
+    mean_mode_block<T>(spec, lstride, nz, prof, prof_stride, transpose, tri_smem());
+    return;
+  }
+  double(*sh)[3][SEG_COLS] = reinterpret_cast<double(*)[3][SEG_COLS]>(tri_smem());  // [segment]: end value, factor
+  const int c = threadIdx.x & (SEG_COLS - 1), g = threadIdx.x / SEG_COLS, ng = blockDim.x / SEG_COLS;
+  const long long col = (long long)blockIdx.x * SEG_COLS + c;
+  const bool in = col < (long long)ny * ncols;
+  const int ky = in ? (int)(col / ncols) : 0, cc = in ? (int)(col - (long long)ky * ncols) : 0, kx = kx0 + cc;
+  const bool on = in && !(kx == 0 && ky == 0);  // the mean mode's column is the extra block's
+  C* sp = spec + spec_row(ky, 1, rpb, ncols, nz) + cc;
+  const int kyi = ky <= ny / 2 ? ky : ny - ky;
+  const long long bstride = (long long)(ny / 2 + 1) * nxh;
+  const double* __restrict__ bcol = b1 + (long long)kyi * nxh + kx;
+  const int k0 = 2 + g * LV;  // this thread's levels k0 .. k0+LV-1, those above nz left out
+  double re[LV], im[LV], b[LV], f[LV];
+  double bprev = 0.0;
+  if (on && k0 >= 3) bprev = __ldg(bcol + (long long)(k0 - 1) * bstride);
+#pragma unroll
+  for (int q = 0; q < LV; ++q) {
+    const int k = k0 + q;
+    re[q] = im[q] = b[q] = 0.0;
+    if (on && k <= nz) {
+      const C v = sp[(long long)(k - 1) * lstride];
+      re[q] = (double)v.x;
+      im[q] = (double)v.y;
+      b[q] = __ldg(bcol + (long long)k * bstride);
+    }
+  }
+  // forward elimination s(k) = d(k) - lo(k) b1(k-1) s(k-1), s(2) = d(2)
+  double er = 0.0, ei = 0.0, fac = 1.0;
+#pragma unroll
+  for (int q = 0; q < LV; ++q) {
+    const int k = k0 + q;
+    f[q] = k >= 3 && k <= nz ? (transpose ? cza[k - 1] : czb[k]) * (q == 0 ? bprev : b[q - 1]) : 0.0;
+    if (k <= nz) {
+      er = re[q] - f[q] * er;
+      ei = im[q] - f[q] * ei;
+      fac = -f[q] * fac;
+    }
+  }
+  sh[g][0][c] = er;
+  sh[g][1][c] = ei;
+  sh[g][2][c] = fac;
+  __syncthreads();
+  double sr = 0.0, si = 0.0;
+  for (int q = 0; q < g; ++q) {
+    sr = sh[q][0][c] + sh[q][2][c] * sr;
+    si = sh[q][1][c] + sh[q][2][c] * si;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int q = 0; q < LV; ++q)
+    if (k0 + q <= nz) {
+      sr = re[q] - f[q] * sr;
+      si = im[q] - f[q] * si;
+      re[q] = sr * b[q];  // e(k) = s(k) b1(k)
+      im[q] = si * b[q];
+    }
+  // back substitution p(k) = e(k) - up(k) b1(k) p(k+1), p(nz) = e(nz)
+  er = ei = 0.0;
+  fac = 1.0;
+#pragma unroll
+  for (int q = LV - 1; q >= 0; --q) {
+    const int k = k0 + q;
+    f[q] = k < nz ? (transpose ? czb[k + 1] : cza[k]) * b[q] : 0.0;
+    if (k <= nz) {
+      er = re[q] - f[q] * er;
+      ei = im[q] - f[q] * ei;
+      fac = -f[q] * fac;
+    }
+  }
+  sh[g][0][c] = er;
+  sh[g][1][c] = ei;
+  sh[g][2][c] = fac;
+  __syncthreads();
+  double pr = 0.0, pi = 0.0;
+  for (int q = ng - 1; q > g; --q) {
+    pr = sh[q][0][c] + sh[q][2][c] * pr;
+    pi = sh[q][1][c] + sh[q][2][c] * pi;
+  }
+#pragma unroll
+  for (int q = LV - 1; q >= 0; --q) {
+    const int k = k0 + q;
+    if (on && k <= nz) {
+      pr = re[q] - f[q] * pr;
+      pi = im[q] - f[q] * pi;
+      C o;
+      o.x = (T)pr;
+      o.y = (T)pi;
+      sp[(long long)(k - 1) * lstride] = o;
+    }
+  }
+}
+
+// Segmented solve or one thread per column?  Columns for fewer than four blocks of 32 per SM, on up
+// to 193 levels (SEG_MAX segments of 12), are too few for the column
+// kernel (64 x 64 x 65 in FP64 4.5 us against 14.2, 128 x 128 x 96 10.5 against 21.6; but 256 x 256 x 128 39.8
+// against 33.5, where the column kernel streams).  The whole grid's
+// columns decide, so that a y-slab's block of them is solved as the single domain solves it.
+static int seg_levels(long long columns, int nz) {
+  const int rows = nz - 1;
+  if (columns > 148LL * 4 * SEG_COLS || rows > 12 * SEG_MAX) return 0;
+  return rows <= 4 * SEG_MAX ? 4 : (rows <= 8 * SEG_MAX ? 8 : 12);
+}
+template <typename T>
+static bool launch_tridiag_seg(typename Cx<T>::t* spec, const double* b1, const double* prof, int prof_stride, int nx, int ny,
+                               int nz, bool transpose, int ncols, int kx0, int rpb, cudaStream_t st) {
+  const long long ncol = (long long)ny * ncols;
+  const int lv = seg_levels((long long)ny * (nx / 2 + 1), nz);
+  if (lv == 0) return false;
+  const int segs = (nz - 1 + lv - 1) / lv;
+  const unsigned grid = (unsigned)((ncol + SEG_COLS - 1) / SEG_COLS + (kx0 == 0 ? 1 : 0));
+  const size_t chain = (size_t)segs * 3 * SEG_COLS * sizeof(double), mean = mean_smem(nz);
+  const size_t smem = chain > mean ? chain : mean;  // at most 12.3 KB
+  const int t = transpose ? 1 : 0;
+  if (lv == 4) k_tridiag_seg<T, 4><<<grid, SEG_COLS * segs, smem, st>>>(spec, b1, prof, prof_stride, nx, ny, nz, t, ncols, kx0, rpb);
+  else if (lv == 8) k_tridiag_seg<T, 8><<<grid, SEG_COLS * segs, smem, st>>>(spec, b1, prof, prof_stride, nx, ny, nz, t, ncols, kx0, rpb);
+  else k_tridiag_seg<T, 12><<<grid, SEG_COLS * segs, smem, st>>>(spec, b1, prof, prof_stride, nx, ny, nz, t, ncols, kx0, rpb);
+  return true;
+}
+
 // The column solve of ncols kx columns (global kx0 ..) on ny rows
 template <typename T>
 static void launch_tridiag(typename Cx<T>::t* spec, double2* s1, const double* b1, const double* prof, int prof_stride,
                            int nx, int ny, int nz, bool transpose, int ncols, int kx0, int rpb, cudaStream_t st) {
   typedef typename Cx<T>::t C;
   const long long ncol = (long long)ny * ncols;
+  if (launch_tridiag_seg<T>(spec, b1, prof, prof_stride, nx, ny, nz, transpose, ncols, kx0, rpb, st)) return;
   ensure_tri_attr();
   k_tridiag<T><<<(unsigned)((ncol + TRI_TB - 1) / TRI_TB + (kx0 == 0 ? 1 : 0)), TRI_TB, tri_smem_bytes<C>(nz), st>>>(
       spec, s1, b1, prof, prof_stride, nx, ny, nz, transpose ? 1 : 0, ncols, kx0, rpb);
@@ -1688,9 +1829,7 @@ extern "C" int mgpu_poisson_fft_noalloc(double* p, int32_t nx, int32_t ny, int32
   // the five solve kernels of fft_solve, on the scratch buffers
   launch_fft_x<double>(false, nx, p, spec, twx, ny, nz, ny, 0, 1, st);
   launch_fft_y<double>(false, ny, spec, twy, nxh, nz, ny, st);
-  ensure_tri_attr();
-  k_tridiag<double><<<(unsigned)((plane + TRI_TB - 1) / TRI_TB + 1), TRI_TB, tri_smem_bytes<double2>(nz), st>>>(
-      spec, s1, b1, prof, stride, nx, ny, nz, 0, nxh, 0, ny);
+  launch_tridiag<double>(spec, s1, b1, prof, stride, nx, ny, nz, false, nxh, 0, ny, st);
   launch_fft_y<double>(true, ny, spec, twy, nxh, nz, ny, st);
   launch_fft_x<double>(true, nx, p, spec, twx, ny, nz, ny, 0, 1, st);
   const cudaError_t e = cudaGetLastError();

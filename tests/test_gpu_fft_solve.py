@@ -56,3 +56,21 @@ def test_deep_fp32_solve_tracks_fp64_and_repeats_exactly(gpu_lib, adjoint):
     outs64 = solve(c64, rhs, repeats=4, adjoint=adjoint)
     for o in outs64:
         np.testing.assert_array_equal(o, ref)
+
+
+@pytest.mark.parametrize("nz", [4, 5, 6, 9, 65, 66, 129, 130, 192, 193, 194])
+def test_segmented_columns(gpu_lib, nz):
+    """Columns cut into segments of 4, 8 and 12 levels, full and partly filled, and (above 193 levels) not
+    cut: the solve against the oracle, its transpose by the dot-product identity."""
+    c, rhs = setup(16, 36, nz, cf.FP64)
+    o = po.Oracle(c)
+    o.set(api.FIELDS["p"], rhs)
+    o.component(api.COMPONENTS["fftsolver"])
+    ref = o.get(api.FIELDS["p"])
+    got = solve(c, rhs)[0]
+    assert np.abs(got - ref).max() <= 1e-11 * np.abs(ref).max()
+    y = ini.uniform_noise(rhs.shape, 18, 4, 1e-3)
+    y[0] = 0.0
+    aty = solve(c, y, adjoint=True)[0]
+    lhs, r = float(np.vdot(got, y)), float(np.vdot(rhs, aty))
+    assert abs(lhs - r) <= 1e-10 * float(np.linalg.norm(got) * np.linalg.norm(y))
