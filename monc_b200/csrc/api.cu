@@ -715,6 +715,17 @@ static int cfltest_callback(mgpu_handle* h, bool evaluate) {
   return MGPU_OK;
 }
 
+// The mean profiles of a step after its dynamics and the swap of the scalar buffers: u + ugal, v + vgal
+// (stepfields.F90 adds the Galilean velocity before the solver group) and the old theta and q,
+// time-smoothed on a centred step; the swap left the old th, zth, q, zq in th_n, zth_n, q_n, zq_n
+template <typename T>
+static int step_mean_profiles(mgpu_handle* h, const DevState<T>& d, int halo) {
+  const bool fwd = h->sc.forward != 0;
+  const MeanProfileFields<T> f{d.zu_n, d.zv_n, d.th, d.q, d.u, d.v, d.th_n, fwd ? nullptr : d.zth_n, d.q_n,
+                               fwd ? nullptr : d.zq_n, h->sc.ugal, h->sc.vgal, 1.0 - 2.0 * h->sc.tsmth, h->sc.tsmth};
+  return launch_mean_profiles<T>(h->sc, f, h->olz_d, h->olbar_d, h->stream, halo);
+}
+
 template <typename T>
 static int step_once(mgpu_handle* h, DevState<T>& d) {
   const bool cfl = h->cfg.cfl_enabled != 0;
@@ -757,14 +768,7 @@ static int step_once(mgpu_handle* h, DevState<T>& d) {
   swap_scalar_buffers<T>(d, h->cfg.number_q_fields);
   // mean_profiles (solver group): the stepped zu, zv and the new theta, q before the pressure step
   if (needs_mean_profiles(h->cfg)) {
-    h->launches += launch_mean_profiles<T>(h->sc, d.zu_n, d.zv_n, d.th, d.q, h->olz_d, h->stream);
-    // u + ugal, v + vgal (stepfields.F90 adds the Galilean velocity before the solver group) and
-    // the old theta and q, time-smoothed on a centred step; the swap left the old th, zth, q, zq
-    // in th_n, zth_n, q_n, zq_n
-    const bool fwd = h->sc.forward != 0;
-    h->launches += launch_mean_profiles_state<T>(h->sc, d.u, d.v, d.th_n, fwd ? nullptr : d.zth_n, d.q_n,
-                                                 fwd ? nullptr : d.zq_n, h->sc.ugal, h->sc.vgal,
-                                                 1.0 - 2.0 * h->sc.tsmth, h->sc.tsmth, h->olbar_d, h->stream);
+    h->launches += step_mean_profiles<T>(h, d, 0);
   }
   // The FFT solve forms the source inside its first transform (fast build); the reproducible build
   // keeps the source kernel, whose rounding the oracle matches.
@@ -980,9 +984,9 @@ static int component(mgpu_handle* h, DevState<T>& d, int cid) {
     case MGPU_C_STEPPING_DIRECTION: return MGPU_OK;
     case MGPU_C_MEAN_PROFILES:
       // the component fields already hold u + ugal and the time-smoothed theta, as MONC's do
-      h->launches += launch_mean_profiles<T>(h->sc, d.zu, d.zv, d.zth, d.zq, h->olz_d, h->stream);
-      h->launches += launch_mean_profiles_state<T>(h->sc, d.u, d.v, d.th, nullptr, d.q, nullptr, 0.0, 0.0, 1.0, 0.0,
-                                                   h->olbar_d, h->stream);
+      h->launches += launch_mean_profiles<T>(
+          h->sc, MeanProfileFields<T>{d.zu, d.zv, d.zth, d.zq, d.u, d.v, d.th, nullptr, d.q, nullptr, 0.0, 0.0, 1.0, 0.0},
+          h->olz_d, h->olbar_d, h->stream);
       break;
     case MGPU_C_FORCING:
       h->launches += subsidence_tendencies(h);
@@ -1360,12 +1364,7 @@ static int step_phase(mgpu_handle* h, DevState<T>& d, int phase) {
       swap_scalar_buffers<T>(d, h->cfg.number_q_fields);
       if (needs_mean_profiles(h->cfg)) {
         // this slab's means; the driver averages them across the slabs (mgpu_slab_mean_profiles)
-        const bool fwd = h->sc.forward != 0;
-        h->launches += launch_mean_profiles<T>(h->sc, d.zu_n, d.zv_n, d.th, d.q, h->olz_d, h->stream, h->slab_halo);
-        h->launches += launch_mean_profiles_state<T>(h->sc, d.u, d.v, d.th_n, fwd ? nullptr : d.zth_n, d.q_n,
-                                                     fwd ? nullptr : d.zq_n, h->sc.ugal, h->sc.vgal,
-                                                     1.0 - 2.0 * h->sc.tsmth, h->sc.tsmth, h->olbar_d, h->stream,
-                                                     h->slab_halo);
+        h->launches += step_mean_profiles<T>(h, d, h->slab_halo);
       }
       if (exact_k) exact::launch_fused_pressure_source<T>(h->sc, d, h->stream);
       else fast::launch_fused_pressure_source<T>(h->sc, d, h->stream);

@@ -110,19 +110,25 @@ int launch_cfl_max_form(const double* src, double* dst, cudaStream_t st);
 template <typename T>
 int launch_divmax(const Scalars& s, const DevState<T>& d, unsigned long long* out, cudaStream_t st, int halo = 0);
 
-// mean profiles (olzubar, olzvbar, olzthbar, olzqbar) of zu, zv, th and q into olz (rows of nz+2),
-// and the mean-profile subsidence tendencies (forcing.cu)
+// the mean profiles (forcing.cu) in one launch: olzubar, olzvbar, olzthbar, olzqbar from zu, zv, the
+// scalar zs and zqs into olz (rows of nz+2); olubar, olvbar, olthbar, olqbar(n) from u + ugal, v + vgal,
+// theta and the q fields (q may be null: no olqbar) into olbar, the scalars after time smoothing
+// c1 f + c2 zf where zth, zq are given
 template <typename T>
-int launch_mean_profiles(const Scalars& s, const T* zu, const T* zv, const T* th, const T* const* q, double* olz,
-                         cudaStream_t st, int halo = 0);
+struct MeanProfileFields {
+  const T *zu, *zv, *zs;
+  const T* const* zqs;
+  const T *u, *v, *th, *zth;
+  const T* const* q;
+  const T* const* zq;
+  double ugal, vgal, c1, c2;
+};
+template <typename T>
+int launch_mean_profiles(const Scalars& s, const MeanProfileFields<T>& f, double* olz, double* olbar, cudaStream_t st,
+                         int halo = 0);
+// the mean-profile subsidence tendencies (forcing.cu)
 int launch_subsidence_tendencies(const Scalars& s, const double* olz, double* tend, bool flow_theta, bool q,
                                  cudaStream_t st);
-// olubar, olvbar, olthbar, olqbar(n) from u, v, theta and the q fields (q may be null: no olqbar);
-// zth, zq given: the scalars after time smoothing c1 f + c2 zf
-template <typename T>
-int launch_mean_profiles_state(const Scalars& s, const T* u, const T* v, const T* th, const T* zth,
-                               const T* const* q, const T* const* zq, double ugal, double vgal, double c1, double c2,
-                               double* olbar, cudaStream_t st, int halo = 0);
 // profile_diagnostics sums into out (MGPU_PD_* rows of nz); qv, ql null for a dry model.  With halo
 // > 0 (a y-slab) the means and sums run over the interior rows halo .. ny-1-halo
 template <typename T>
