@@ -393,6 +393,10 @@ static void state_ptrs(DevState<double>& d, double* out[8]) {
   double* p[8] = {d.u, d.v, d.w, d.th, d.zu, d.zv, d.zw, d.zth};
   for (int q = 0; q < 8; ++q) out[q] = p[q];
 }
+static void set_state_ptrs(DevState<double>& d, double* const* in) {
+  double** p[8] = {&d.u, &d.v, &d.w, &d.th, &d.zu, &d.zv, &d.zw, &d.zth};
+  for (int q = 0; q < 8; ++q) *p[q] = in[q];
+}
 
 static int ad_alloc(mgpu_handle* h, double** p, size_t n) {
   if (cudaMalloc((void**)p, n * sizeof(double)) != cudaSuccess) return fail(h, MGPU_ERR_CUDA, "cudaMalloc (adjoint work)");
@@ -856,11 +860,12 @@ static void copy_state(mgpu_handle* h, double* const* dst, double* const* src) {
   for (int q = 0; q < 8; ++q) cudaMemcpyAsync(dst[q], src[q], bytes, cudaMemcpyDeviceToDevice, h->stream);
 }
 
-// the adjoint of one step from state X (already in h->d64): adjoints of the next state in
-// adj[cur] become adjoints of X in adj[1-cur]
-static int adjoint_step(mgpu_handle* h) {
+// the adjoint of one step from the state X: adjoints of the next state in adj[cur] become adjoints
+// of X in adj[1-cur].  X's arrays stand in for the model's; the recomputation changes their surface level
+static int adjoint_step(mgpu_handle* h, double* const* X) {
   AdWork* a = h->ad;
-  DevState<double>& d = h->d64;
+  DevState<double> d = h->d64;
+  set_state_ptrs(d, X);
   h->sc.forward = (h->timestep == 1) ? 1 : 0;
   // recompute the step's intermediates.  The hand-written passes read only the step's input state
   // (with lower_bc's th(1) or zth(1)) and vis, diff: the pressure step and source are linear and
@@ -876,8 +881,10 @@ static int adjoint_step(mgpu_handle* h) {
   double* const* B = a->adj[a->cur];
   double* const* A = a->adj[1 - a->cur];
   const size_t bytes = field_elems(h) * sizeof(double);
-  for (int q = 0; q < 8; ++q) CK(cudaMemsetAsync(A[q], 0, bytes, h->stream));
-  for (int q = 0; q < 6; ++q) CK(cudaMemsetAsync(a->inter[q], 0, bytes, h->stream));
+  if (h->cfg.adjoint_taped) {  // the hand-written pass 4 sets all of them
+    for (int q = 0; q < 8; ++q) CK(cudaMemsetAsync(A[q], 0, bytes, h->stream));
+    for (int q = 0; q < 6; ++q) CK(cudaMemsetAsync(a->inter[q], 0, bytes, h->stream));
+  }
   double* tg[F_COUNT];
   for (int q = 0; q < 8; ++q) tg[F_U + q] = A[q];
   tg[F_VIS] = a->inter[0];
@@ -925,41 +932,48 @@ static int adjoint_run(mgpu_handle* h, int nsteps, int interval, double* rmlmax_
     a->seg.push_back(p);
   }
   double* X[8];
-  // forward sweep, saving a checkpoint every `interval` steps
+  // forward sweep, saving a checkpoint every `interval` steps and each input state of the last segment,
+  // which the reverse sweep starts with
+  const int last = (nck - 1) * interval;
   for (int st = 0; st < nsteps; ++st) {
     state_ptrs(d, X);
-    if (st % interval == 0) copy_state(h, &a->ckpt[8 * (st / interval)], X);
+    if (st >= last) copy_state(h, &a->seg[8 * (st - last)], X);
+    else if (st % interval == 0) copy_state(h, &a->ckpt[8 * (st / interval)], X);
     int rc = step_once<double>(h, d);
     if (rc) return rc;
   }
-  state_ptrs(d, X);
-  copy_state(h, a->final_state, X);
+  if (nck > 1) {  // recomputing the earlier segments overwrites the state
+    state_ptrs(d, X);
+    copy_state(h, a->final_state, X);
+  }
   CK(cudaMemsetAsync(a->prof_bar, 0, (h->cfg.nz + 2) * sizeof(double), h->stream));
   CK(cudaMemsetAsync(a->overflow, 0, sizeof(int), h->stream));
   // reverse sweep, one checkpoint segment at a time
   for (int c = nck - 1; c >= 0; --c) {
     const int s0 = c * interval, s1 = std::min(nsteps, s0 + interval);
-    state_ptrs(d, X);
-    copy_state(h, X, &a->ckpt[8 * c]);
-    h->timestep = t0 + s0;
-    // the input states of steps s0 .. s1-1; the last step's own result is not needed
-    for (int st = s0; st < s1; ++st) {
+    if (c < nck - 1) {
+      // the input states of steps s0 .. s1-1; the last step's own result is not needed
       state_ptrs(d, X);
-      copy_state(h, &a->seg[8 * (st - s0)], X);
-      if (st == s1 - 1) break;
-      int rc = step_once<double>(h, d);
-      if (rc) return rc;
+      copy_state(h, X, &a->ckpt[8 * c]);
+      h->timestep = t0 + s0;
+      for (int st = s0;; ++st) {
+        state_ptrs(d, X);
+        copy_state(h, &a->seg[8 * (st - s0)], X);
+        if (st == s1 - 1) break;
+        int rc = step_once<double>(h, d);
+        if (rc) return rc;
+      }
     }
     for (int st = s1 - 1; st >= s0; --st) {
-      state_ptrs(d, X);
-      copy_state(h, X, &a->seg[8 * (st - s0)]);
       h->timestep = t0 + st;
-      int rc = adjoint_step(h);
+      int rc = adjoint_step(h, &a->seg[8 * (st - s0)]);
       if (rc) return rc;
     }
   }
-  state_ptrs(d, X);
-  copy_state(h, X, a->final_state);
+  if (nck > 1) {
+    state_ptrs(d, X);
+    copy_state(h, X, a->final_state);
+  }
   h->timestep = t0 + nsteps;
   int ovf = 0;
   std::vector<double> pb(h->cfg.nz + 2);
