@@ -6,13 +6,16 @@
 //     their adjoints are written in gather form: each thread forms the adjoint of its own inputs
 //     from the output adjoints of the points that read them, with no atomics;
 //   * momentum (PW advection, viscosity, Coriolis, buoyancy, stepping) is a bilinear stencil; its
-//     adjoint is written in scatter form: each thread evaluates the partial derivatives of its
-//     outputs in registers, sums the contributions that land on the same input point, and adds
-//     them into the input adjoints with FP64 atomics.
+//     adjoint, and the subgrid pass's, is written in scatter form: each thread evaluates the partial
+//     derivatives of its outputs in registers, and the contributions that land on the same input point
+//     are summed over the thread, its row and its tile before one FP64 atomic adds them to the input
+//     adjoint (adjoint_rows.cuh);
+//   * the scalar pass adds its limiter's data-dependent stencil point by point with FP64 atomics.
 // The adjoint arrays and seeds follow adj_pass (tlad.cu); the operator-overloading tape kernels
 // there evaluate the same transposes and are the check these kernels are tested against.
 #include "dycore.h"
 #include "dycore_device.cuh"
+#include "adjoint_rows.cuh"
 
 namespace mgpu {
 namespace hadj {
@@ -136,86 +139,99 @@ __global__ void __launch_bounds__(128) k_hadj_pressure_source(Scalars s, Args a)
 }
 
 // ---- momentum (eval_momentum: pw_point, viscosity_point, coriolis_point, buoyancy, stepping) ---
-struct VelAdj {
-  int fu, fv, fw;  // adjoint targets of ZU, ZV, ZW (u, v, w on the forward step, else zu, zv, zw)
+// what a point adds to the velocities and the viscosity around it
+struct VelCells {
+  Cells u, v, w, vis;
 };
+// vb to the four columns from (dj, di) on, of levels k - 1 and k
+__device__ __forceinline__ void add_box(Cells& x, int dj, int di, double vb) {
+#pragma unroll
+  for (int dk = -1; dk <= 0; ++dk)
+#pragma unroll
+    for (int q = 0; q < 4; ++q) x.add(dk, dj + (q >> 1), di + (q & 1), vb);
+}
 
-// adjoint of tau_13_23(kk) (the t13, t13m1, t23, t23m1 stresses) with the given bars
+// adjoint of tau_13_23(kk), kk = k + DK (the t13, t23 and with M1 the t13m1, t23m1 stresses) with the
+// given bars
+template <int DK, bool M1>
 __device__ __forceinline__ void adj_tau13_23(const Scalars& s, const Prof<double>& P, const View<double>& ZU,
                                              const View<double>& ZV, const View<double>& ZW,
-                                             const View<double>& VIS, const Scatter& S, const VelAdj& f, int kk,
-                                             int j, int i, double b13, double b13m1, double b23, double b23m1) {
+                                             const View<double>& VIS, VelCells& A, int k, int j, int i, double b13, double b13m1, double b23, double b23m1) {
+  const int kk = k + DK;
   const double cx = s.cx, cy = s.cy, rdzn = P(P_RDZN, kk + 1), rho = P(P_RHO, kk);
-  if (b13 != 0.0) {
+  {
     const double vis13 = 0.5 * (VIS(kk, j, i) + VIS(kk, j, i + 1));
     const double gr = (ZU(kk + 1, j, i) - ZU(kk, j, i)) * rdzn + (ZW(kk, j, i + 1) - ZW(kk, j, i)) * cx;
     const double gb = b13 * rho * vis13, vb = 0.5 * b13 * gr * rho;
-    S(f.fu, kk + 1, j, i, gb * rdzn);
-    S(f.fu, kk, j, i, -gb * rdzn);
-    S(f.fw, kk, j, i + 1, gb * cx);
-    S(f.fw, kk, j, i, -gb * cx);
-    S(F_VIS, kk, j, i, vb);
-    S(F_VIS, kk, j, i + 1, vb);
+    A.u.add(DK + 1, 0, 0, gb * rdzn);
+    A.u.add(DK, 0, 0, -gb * rdzn);
+    A.w.add(DK, 0, 1, gb * cx);
+    A.w.add(DK, 0, 0, -gb * cx);
+    A.vis.add(DK, 0, 0, vb);
+    A.vis.add(DK, 0, 1, vb);
   }
-  if (b13m1 != 0.0) {
+  if (M1) {
     const double vis13 = 0.5 * (VIS(kk, j, i - 1) + VIS(kk, j, i));
     const double gr = (ZU(kk + 1, j, i - 1) - ZU(kk, j, i - 1)) * rdzn + (ZW(kk, j, i) - ZW(kk, j, i - 1)) * cx;
     const double gb = b13m1 * rho * vis13, vb = 0.5 * b13m1 * gr * rho;
-    S(f.fu, kk + 1, j, i - 1, gb * rdzn);
-    S(f.fu, kk, j, i - 1, -gb * rdzn);
-    S(f.fw, kk, j, i, gb * cx);
-    S(f.fw, kk, j, i - 1, -gb * cx);
-    S(F_VIS, kk, j, i - 1, vb);
-    S(F_VIS, kk, j, i, vb);
+    A.u.add(DK + 1, 0, -1, gb * rdzn);
+    A.u.add(DK, 0, -1, -gb * rdzn);
+    A.w.add(DK, 0, 0, gb * cx);
+    A.w.add(DK, 0, -1, -gb * cx);
+    A.vis.add(DK, 0, -1, vb);
+    A.vis.add(DK, 0, 0, vb);
   }
-  if (b23 != 0.0) {
+  {
     const double vis23 = 0.5 * (VIS(kk, j, i) + VIS(kk, j + 1, i));
     const double gr = (ZW(kk, j + 1, i) - ZW(kk, j, i)) * cy + (ZV(kk + 1, j, i) - ZV(kk, j, i)) * rdzn;
     const double gb = b23 * rho * vis23, vb = 0.5 * b23 * gr * rho;
-    S(f.fw, kk, j + 1, i, gb * cy);
-    S(f.fw, kk, j, i, -gb * cy);
-    S(f.fv, kk + 1, j, i, gb * rdzn);
-    S(f.fv, kk, j, i, -gb * rdzn);
-    S(F_VIS, kk, j, i, vb);
-    S(F_VIS, kk, j + 1, i, vb);
+    A.w.add(DK, 1, 0, gb * cy);
+    A.w.add(DK, 0, 0, -gb * cy);
+    A.v.add(DK + 1, 0, 0, gb * rdzn);
+    A.v.add(DK, 0, 0, -gb * rdzn);
+    A.vis.add(DK, 0, 0, vb);
+    A.vis.add(DK, 1, 0, vb);
   }
-  if (b23m1 != 0.0) {
+  if (M1) {
     const double vis23 = 0.5 * (VIS(kk, j - 1, i) + VIS(kk, j, i));
     const double gr = (ZW(kk, j, i) - ZW(kk, j - 1, i)) * cy + (ZV(kk + 1, j - 1, i) - ZV(kk, j - 1, i)) * rdzn;
     const double gb = b23m1 * rho * vis23, vb = 0.5 * b23m1 * gr * rho;
-    S(f.fw, kk, j, i, gb * cy);
-    S(f.fw, kk, j - 1, i, -gb * cy);
-    S(f.fv, kk + 1, j - 1, i, gb * rdzn);
-    S(f.fv, kk, j - 1, i, -gb * rdzn);
-    S(F_VIS, kk, j - 1, i, vb);
-    S(F_VIS, kk, j, i, vb);
+    A.w.add(DK, 0, 0, gb * cy);
+    A.w.add(DK, -1, 0, -gb * cy);
+    A.v.add(DK + 1, -1, 0, gb * rdzn);
+    A.v.add(DK, -1, 0, -gb * rdzn);
+    A.vis.add(DK, -1, 0, vb);
+    A.vis.add(DK, 0, 0, vb);
   }
 }
 
-// adjoint of tau33_at(kk) = rhon(kk) (vis(kk) + vis(kk-1)) (zw(kk) - zw(kk-1)) rdz(kk)
+// adjoint of tau33_at(kk) = rhon(kk) (vis(kk) + vis(kk-1)) (zw(kk) - zw(kk-1)) rdz(kk), kk = k + DK
+template <int DK>
 __device__ __forceinline__ void adj_tau33(const Prof<double>& P, const View<double>& ZW, const View<double>& VIS,
-                                          const Scatter& S, int fw, int kk, int j, int i, double b) {
-  if (kk <= 1 || b == 0.0) return;
+                                          VelCells& A, int k, int j, int i, double b) {
+  const int kk = k + DK;  // >= 2
   const double rhon = P(P_RHON, kk), rdz = P(P_RDZ, kk);
   const double visonp2 = rhon * (VIS(kk, j, i) + VIS(kk - 1, j, i));
   const double dw = (ZW(kk, j, i) - ZW(kk - 1, j, i));
-  S(fw, kk, j, i, b * visonp2 * rdz);
-  S(fw, kk - 1, j, i, -b * visonp2 * rdz);
+  A.w.add(DK, 0, 0, b * visonp2 * rdz);
+  A.w.add(DK - 1, 0, 0, -b * visonp2 * rdz);
   const double vb = b * rhon * dw * rdz;
-  S(F_VIS, kk, j, i, vb);
-  S(F_VIS, kk - 1, j, i, vb);
+  A.vis.add(DK, 0, 0, vb);
+  A.vis.add(DK - 1, 0, 0, vb);
 }
 
-// adjoint of viscosity_point with the bars du_b, dv_b, dw_b of its three increments
-__device__ void adj_viscosity(const Scalars& s, const Prof<double>& P, const View<double>& ZU,
+// adjoint of viscosity_point with the bars du_b, dv_b, dw_b of its three increments, but for what it adds
+// to zu at x+1, which it returns
+__device__ __forceinline__ double adj_viscosity(const Scalars& s, const Prof<double>& P, const View<double>& ZU,
                               const View<double>& ZV, const View<double>& ZW, const View<double>& ZUs,
-                              const View<double>& VIS, const Scatter& S, const VelAdj& f, int k, int j, int i,
+                              const View<double>& VIS, VelCells& A, int k, int j, int i,
                               double du_b, double dv_b, double dw_b) {
   const double cx = s.cx, cy = s.cy, rhon = P(P_RHON, k);
   const double xa = s.rho_unity ? du_b : du_b / rhon;
   const double xb = s.rho_unity ? dv_b : dv_b / rhon;
   const double xc = (k < s.nz) ? (s.rho_unity ? dw_b : dw_b / P(P_RHO, k)) : 0.0;
   const double rdz = P(P_RDZ, k);
+  double zu_e;
   // bars of the stresses the three increments difference
   const double b11p1 = xa * cx, b11 = -xa * cx;
   const double b12 = xa * cy + xb * cx, b12ym1 = -xa * cy, b12m1 = -xb * cx;
@@ -227,13 +243,11 @@ __device__ void adj_viscosity(const Scalars& s, const Prof<double>& P, const Vie
                                   VIS(k, j, i + 1) + VIS(k, j + 1, i + 1) + VIS(k - 1, j, i + 1) +
                                   VIS(k - 1, j + 1, i + 1));
     const double gb = b12 * rhon * vis12, vb = 0.125 * b12 * gr * rhon;
-    S(f.fu, k, j + 1, i, gb * cy);
-    S(f.fu, k, j, i, -gb * cy);
-    S(f.fv, k, j, i + 1, gb * cx);
-    S(f.fv, k, j, i, -gb * cx);
-    for (int kk = k - 1; kk <= k; ++kk)
-      for (int jj = j; jj <= j + 1; ++jj)
-        for (int ii = i; ii <= i + 1; ++ii) S(F_VIS, kk, jj, ii, vb);
+    A.u.add(0, 1, 0, gb * cy);
+    A.u.add(0, 0, 0, -gb * cy);
+    A.v.add(0, 0, 1, gb * cx);
+    A.v.add(0, 0, 0, -gb * cx);
+    add_box(A.vis, 0, 0, vb);
   }
   // tau12m1: columns i-1, i of rows j, j+1
   {
@@ -242,13 +256,11 @@ __device__ void adj_viscosity(const Scalars& s, const Prof<double>& P, const Vie
                                   VIS(k, j, i - 1) + VIS(k, j + 1, i - 1) + VIS(k - 1, j, i - 1) +
                                   VIS(k - 1, j + 1, i - 1));
     const double gb = b12m1 * rhon * vis12, vb = 0.125 * b12m1 * gr * rhon;
-    S(f.fu, k, j + 1, i - 1, gb * cy);
-    S(f.fu, k, j, i - 1, -gb * cy);
-    S(f.fv, k, j, i, gb * cx);
-    S(f.fv, k, j, i - 1, -gb * cx);
-    for (int kk = k - 1; kk <= k; ++kk)
-      for (int jj = j; jj <= j + 1; ++jj)
-        for (int ii = i - 1; ii <= i; ++ii) S(F_VIS, kk, jj, ii, vb);
+    A.u.add(0, 1, -1, gb * cy);
+    A.u.add(0, 0, -1, -gb * cy);
+    A.v.add(0, 0, 0, gb * cx);
+    A.v.add(0, 0, -1, -gb * cx);
+    add_box(A.vis, 0, -1, vb);
   }
   // tau12_ym1: columns i, i+1 of rows j-1, j
   {
@@ -257,60 +269,60 @@ __device__ void adj_viscosity(const Scalars& s, const Prof<double>& P, const Vie
                                   VIS(k, j - 1, i + 1) + VIS(k, j, i + 1) + VIS(k - 1, j - 1, i + 1) +
                                   VIS(k - 1, j, i + 1));
     const double gb = b12ym1 * rhon * vis12, vb = 0.125 * b12ym1 * gr * rhon;
-    S(f.fu, k, j, i, gb * cy);
-    S(f.fu, k, j - 1, i, -gb * cy);
-    S(f.fv, k, j - 1, i + 1, gb * cx);
-    S(f.fv, k, j - 1, i, -gb * cx);
-    for (int kk = k - 1; kk <= k; ++kk)
-      for (int jj = j - 1; jj <= j; ++jj)
-        for (int ii = i; ii <= i + 1; ++ii) S(F_VIS, kk, jj, ii, vb);
+    A.u.add(0, 0, 0, gb * cy);
+    A.u.add(0, -1, 0, -gb * cy);
+    A.v.add(0, -1, 1, gb * cx);
+    A.v.add(0, -1, 0, -gb * cx);
+    add_box(A.vis, -1, 0, vb);
   }
   // tau11 and tau22 share visonp2 = rhon (vis(k) + vis(k-1)) at (j, i)
   {
     const double visonp2 = rhon * (VIS(k, j, i) + VIS(k - 1, j, i));
     const double du = (ZU(k, j, i) - ZU(k, j, i - 1)), dv = (ZV(k, j, i) - ZV(k, j - 1, i));
-    S(f.fu, k, j, i, b11 * visonp2 * cx);
-    S(f.fu, k, j, i - 1, -b11 * visonp2 * cx);
-    S(f.fv, k, j, i, b22 * visonp2 * cy);
-    S(f.fv, k, j - 1, i, -b22 * visonp2 * cy);
+    A.u.add(0, 0, 0, b11 * visonp2 * cx);
+    A.u.add(0, 0, -1, -b11 * visonp2 * cx);
+    A.v.add(0, 0, 0, b22 * visonp2 * cy);
+    A.v.add(0, -1, 0, -b22 * visonp2 * cy);
     const double vb = rhon * (b11 * du * cx + b22 * dv * cy);
-    S(F_VIS, k, j, i, vb);
-    S(F_VIS, k - 1, j, i, vb);
+    A.vis.add(0, 0, 0, vb);
+    A.vis.add(-1, 0, 0, vb);
   }
   // tau22_yp1 at (j+1, i)
   {
     const double visonp2 = rhon * (VIS(k, j + 1, i) + VIS(k - 1, j + 1, i));
     const double dv = (ZV(k, j + 1, i) - ZV(k, j, i));
-    S(f.fv, k, j + 1, i, b22yp1 * visonp2 * cy);
-    S(f.fv, k, j, i, -b22yp1 * visonp2 * cy);
+    A.v.add(0, 1, 0, b22yp1 * visonp2 * cy);
+    A.v.add(0, 0, 0, -b22yp1 * visonp2 * cy);
     const double vb = rhon * b22yp1 * dv * cy;
-    S(F_VIS, k, j + 1, i, vb);
-    S(F_VIS, k - 1, j + 1, i, vb);
+    A.vis.add(0, 1, 0, vb);
+    A.vis.add(-1, 1, 0, vb);
   }
   // tau11p1 at (j, i+1): current_state%zu at x+1 minus ZU at x
   {
     const double visonp2 = rhon * (VIS(k, j, i + 1) + VIS(k - 1, j, i + 1));
     const double du = (ZUs(k, j, i + 1) - ZU(k, j, i));
-    S(F_ZU, k, j, i + 1, b11p1 * visonp2 * cx);
-    S(f.fu, k, j, i, -b11p1 * visonp2 * cx);
+    zu_e = b11p1 * visonp2 * cx;
+    A.u.add(0, 0, 0, -b11p1 * visonp2 * cx);
     const double vb = rhon * b11p1 * du * cx;
-    S(F_VIS, k, j, i + 1, vb);
-    S(F_VIS, k - 1, j, i + 1, vb);
+    A.vis.add(0, 0, 1, vb);
+    A.vis.add(-1, 0, 1, vb);
   }
   // vertical stresses
   if (k < s.nz)
-    adj_tau13_23(s, P, ZU, ZV, ZW, VIS, S, f, k, j, i, xa * rdz + xc * cx, -xc * cx, xb * rdz + xc * cy, -xc * cy);
-  adj_tau13_23(s, P, ZU, ZV, ZW, VIS, S, f, k - 1, j, i, -xa * rdz, 0.0, -xb * rdz, 0.0);
+    adj_tau13_23<0, true>(s, P, ZU, ZV, ZW, VIS, A, k, j, i, xa * rdz + xc * cx, -xc * cx, xb * rdz + xc * cy,
+                          -xc * cy);
+  adj_tau13_23<-1, false>(s, P, ZU, ZV, ZW, VIS, A, k, j, i, -xa * rdz, 0.0, -xb * rdz, 0.0);
   if (k < s.nz) {
     const double rdzn1 = P(P_RDZN, k + 1);
-    adj_tau33(P, ZW, VIS, S, f.fw, k + 1, j, i, xc * rdzn1);
-    adj_tau33(P, ZW, VIS, S, f.fw, k, j, i, -xc * rdzn1);
+    adj_tau33<1>(P, ZW, VIS, A, k, j, i, xc * rdzn1);
+    adj_tau33<0>(P, ZW, VIS, A, k, j, i, -xc * rdzn1);
   }
+  return zu_e;
 }
 
 // adjoint of pw_point with the bars a, b, c of su, sv, sw (c = 0 at k = nz, where sw is not set)
-__device__ void adj_pw(const Scalars& s, const Prof<double>& P, const View<double>& U, const View<double>& V,
-                       const View<double>& W, const Scatter& S, int k, int j, int i, double a, double b, double c) {
+__device__ __forceinline__ void adj_pw(const Scalars& s, const Prof<double>& P, const View<double>& U, const View<double>& V,
+                       const View<double>& W, VelCells& A, int k, int j, int i, double a, double b, double c) {
   const double tcx = s.tcx, tcy = s.tcy, tzc1 = P(P_TZC1, k);
   const double u0 = U(k, j, i), v0 = V(k, j, i);
   const double Uw = U(k, j, i - 1), Ue = U(k, j, i + 1), Us = U(k, j - 1, i), Un = U(k, j + 1, i), Ub = U(k - 1, j, i);
@@ -346,84 +358,141 @@ __device__ void adj_pw(const Scalars& s, const Prof<double>& P, const View<doubl
     bv0 += -c * tcy * Wn;
     bvs += c * tcy * Ws;
     bwb += c * tzd1 * (w0 + 2.0 * Wb);
-    S(F_U, k + 1, j, i, -a * tzc2 * (w0 + We) - c * tcx * We);
-    S(F_U, k + 1, j, i - 1, c * tcx * Ww);
-    S(F_V, k + 1, j, i, -b * tzc2 * (w0 + Wn) - c * tcy * Wn);
-    S(F_V, k + 1, j - 1, i, c * tcy * Ws);
-    S(F_W, k, j, i, -a * tzc2 * Ut - b * tzc2 * Vt + c * (tzd1 * Wb - tzd2 * Wt));
-    S(F_W, k, j, i + 1, -a * tzc2 * Ut - c * tcx * (u0 + Ut));
-    S(F_W, k, j + 1, i, -b * tzc2 * Vt - c * tcy * (v0 + Vt));
-    S(F_W, k + 1, j, i, -c * tzd2 * (w0 + 2.0 * Wt));
-    S(F_W, k, j, i - 1, c * tcx * (Uw + Uwt));
-    S(F_W, k, j - 1, i, c * tcy * (Vs + Vst));
+    A.u.add(1, 0, 0, -a * tzc2 * (w0 + We) - c * tcx * We);
+    A.u.add(1, 0, -1, c * tcx * Ww);
+    A.v.add(1, 0, 0, -b * tzc2 * (w0 + Wn) - c * tcy * Wn);
+    A.v.add(1, -1, 0, c * tcy * Ws);
+    A.w.add(0, 0, 0, -a * tzc2 * Ut - b * tzc2 * Vt + c * (tzd1 * Wb - tzd2 * Wt));
+    A.w.add(0, 0, 1, -a * tzc2 * Ut - c * tcx * (u0 + Ut));
+    A.w.add(0, 1, 0, -b * tzc2 * Vt - c * tcy * (v0 + Vt));
+    A.w.add(1, 0, 0, -c * tzd2 * (w0 + 2.0 * Wt));
+    A.w.add(0, 0, -1, c * tcx * (Uw + Uwt));
+    A.w.add(0, -1, 0, c * tcy * (Vs + Vst));
   }
-  S(F_U, k, j, i, bu0);
-  S(F_U, k, j, i - 1, buw);
-  S(F_U, k, j, i + 1, bue);
-  S(F_U, k, j - 1, i, bus);
-  S(F_U, k, j + 1, i, bun);
-  S(F_U, k - 1, j, i, bub);
-  S(F_U, k, j + 1, i - 1, buwn);
-  S(F_V, k, j, i, bv0);
-  S(F_V, k, j, i + 1, bve);
-  S(F_V, k, j - 1, i, bvs);
-  S(F_V, k, j - 1, i + 1, bvse);
-  S(F_V, k, j + 1, i, bvn);
-  S(F_V, k, j, i - 1, bvw);
-  S(F_V, k - 1, j, i, bvb);
-  S(F_W, k - 1, j, i, bwb);
-  S(F_W, k - 1, j, i + 1, bwbe);
-  S(F_W, k - 1, j + 1, i, bwbn);
+  A.u.add(0, 0, 0, bu0);
+  A.u.add(0, 0, -1, buw);
+  A.u.add(0, 0, 1, bue);
+  A.u.add(0, -1, 0, bus);
+  A.u.add(0, 1, 0, bun);
+  A.u.add(-1, 0, 0, bub);
+  A.u.add(0, 1, -1, buwn);
+  A.v.add(0, 0, 0, bv0);
+  A.v.add(0, 0, 1, bve);
+  A.v.add(0, -1, 0, bvs);
+  A.v.add(0, -1, 1, bvse);
+  A.v.add(0, 1, 0, bvn);
+  A.v.add(0, 0, -1, bvw);
+  A.v.add(-1, 0, 0, bvb);
+  A.w.add(-1, 0, 0, bwb);
+  A.w.add(-1, 0, 1, bwbe);
+  A.w.add(-1, 1, 0, bwbn);
 }
 
-__global__ void __launch_bounds__(128) k_hadj_momentum(Scalars s, Args a) {
-  HADJ_POINT_INDEX
-  const double A = a.tg[F_ZUN][o], B = a.tg[F_ZVN][o], C = a.tg[F_ZWN][o];
-  if (A == 0.0 && B == 0.0 && C == 0.0) return;
-  const Geo g = geo(s);
-  const Prof<double> P{s.prof, s.nz + 2};
-  const Scatter S{a.tg, g};
-  const DevState<double>& d = a.d;
+// pw_point and coriolis_point add to U, V, W ...
+constexpr unsigned PW_U = xrow(0, 0) | cell(0, -1, 0) | cell(0, 1, 0) | cell(-1, 0, 0) | cell(0, 1, -1) |
+                          cell(1, 0, 0) | cell(1, 0, -1);
+constexpr unsigned PW_V = xrow(0, 0) | cell(0, -1, 0) | cell(0, -1, 1) | cell(0, 1, 0) | cell(-1, 0, 0) |
+                          cell(1, 0, 0) | cell(1, -1, 0);
+constexpr unsigned PW_W = xrow(0, 0) | cell(0, -1, 0) | cell(0, 1, 0) | cell(1, 0, 0) | cell(-1, 0, 0) |
+                          cell(-1, 0, 1) | cell(-1, 1, 0);
+// ... and viscosity_point to ZU, ZV, ZW and vis
+constexpr unsigned VD_U = xrow(0, 0) | cell(0, 1, 0) | cell(0, -1, 0) | cell(0, 1, -1) | cell(1, 0, 0) |
+                          cell(1, 0, -1) | cell(-1, 0, 0);
+constexpr unsigned VD_V = xrow(0, 0) | cell(0, 1, 0) | cell(0, -1, 0) | cell(0, -1, 1) | cell(1, 0, 0) |
+                          cell(1, -1, 0) | cell(-1, 0, 0);
+constexpr unsigned VD_W = xrow(0, 0) | cell(0, 1, 0) | cell(0, -1, 0) | cell(-1, 0, 0) | cell(-1, 0, 1) |
+                          cell(-1, 1, 0) | cell(1, 0, 0);
+constexpr unsigned VD_VIS = xrow(0, 0) | xrow(0, 1) | cell(0, -1, 0) | cell(0, -1, 1) | xrow(-1, 0) | xrow(-1, 1) |
+                            cell(-1, -1, 0) | cell(-1, -1, 1) | cell(1, 0, 0);
+constexpr int MOM_ROWS = row_count(VD_U) + row_count(VD_V) + row_count(VD_W) + row_count(VD_VIS);
+
+__global__ void __launch_bounds__(HX * HY) k_hadj_momentum(Scalars s, Args a) {
+  __shared__ Rows<MOM_ROWS> sh;
+  const Tile t(s);
+  const Geo g = t.g;
+  const int k = t.k, j = min(t.j, s.ny - 1), i = min(t.i, s.nx - 1);
+  const long long o = (long long)(k - 1) * s.plane + (long long)j * s.nx + i;
+  const double A = t.in ? a.tg[F_ZUN][o] : 0.0, B = t.in ? a.tg[F_ZVN][o] : 0.0, C = t.in ? a.tg[F_ZWN][o] : 0.0;
   const bool fwd = s.forward;
   // stepping: zun = ugal + u + dtm su (forward) or ugal + zu + 2 dtm su (centred)
-  if (fwd) {
-    S(F_U, k, j, i, A);
-    S(F_V, k, j, i, B);
-    S(F_W, k, j, i, C);
-  } else {
-    S(F_ZU, k, j, i, A);
-    S(F_ZV, k, j, i, B);
-    S(F_ZW, k, j, i, C);
+  if (k < 2) {
+    if (!t.in) return;
+    atomicAdd(a.tg[fwd ? F_U : F_ZU] + o, A);
+    atomicAdd(a.tg[fwd ? F_V : F_ZV] + o, B);
+    atomicAdd(a.tg[fwd ? F_W : F_ZW] + o, C);
+    return;
   }
-  if (k < 2) return;
+  const Prof<double> P{s.prof, s.nz + 2};
+  const DevState<double>& d = a.d;
   const double cst = fwd ? s.dtm : 2.0 * s.dtm;
   const double sa = cst * A, sb = cst * B, sc = (k < s.nz) ? cst * C : 0.0;
-  const View<double> U{d.u, g}, V{d.v, g}, W{d.w, g};
-  if (k < s.nz && !s.passive_th) {
+  if (k < s.nz && !s.passive_th && t.in) {
     const double hb = 0.5 * P(P_BUOY_CO, k) * sc;
-    S(F_TH, k, j, i, hb);
-    S(F_TH, k + 1, j, i, hb);
+    atomicAdd(a.tg[F_TH] + o, hb);
+    atomicAdd(a.tg[F_TH] + o + s.plane, hb);
   }
-  if (s.coriolis) {
-    const double q = 0.25 * s.fcoriol * sa, r = -0.25 * s.fcoriol * sb;
-    S(F_V, k, j, i, q);
-    S(F_V, k, j, i + 1, q);
-    S(F_V, k, j - 1, i, q);
-    S(F_V, k, j - 1, i + 1, q);
-    S(F_U, k, j, i, r);
-    S(F_U, k, j, i - 1, r);
-    S(F_U, k, j + 1, i, r);
-    S(F_U, k, j + 1, i - 1, r);
+  {
+    VelCells c;
+    if (s.coriolis) {
+      const double q = 0.25 * s.fcoriol * sa, r = -0.25 * s.fcoriol * sb;
+      c.v.add(0, 0, 0, q);
+      c.v.add(0, 0, 1, q);
+      c.v.add(0, -1, 0, q);
+      c.v.add(0, -1, 1, q);
+      c.u.add(0, 0, 0, r);
+      c.u.add(0, 0, -1, r);
+      c.u.add(0, 1, 0, r);
+      c.u.add(0, 1, -1, r);
+    }
+    if (fwd) {
+      c.u.add(0, 0, 0, A);
+      c.v.add(0, 0, 0, B);
+      c.w.add(0, 0, 0, C);
+    }
+    adj_pw(s, P, View<double>{d.u, g}, View<double>{d.v, g}, View<double>{d.w, g}, c, k, j, i, sa, sb, sc);
+    constexpr int S1 = row_count(PW_U), S2 = S1 + row_count(PW_V);
+    RowSum ru[3], rv[3], rw[3];
+    share_rows<PW_U, 0>(c.u, t, sh, ru);
+    share_rows<PW_V, S1>(c.v, t, sh, rv);
+    share_rows<PW_W, S2>(c.w, t, sh, rw);
+    __syncthreads();
+    add_rows<PW_U, 0>(a.tg[F_U], t, sh, ru);
+    add_rows<PW_V, S1>(a.tg[F_V], t, sh, rv);
+    add_rows<PW_W, S2>(a.tg[F_W], t, sh, rw);
   }
-  if (s.use_vd) {
-    const VelAdj f = fwd ? VelAdj{F_U, F_V, F_W} : VelAdj{F_ZU, F_ZV, F_ZW};
-    const View<double> ZU{fwd ? d.u : d.zu, g}, ZV{fwd ? d.v : d.zv, g}, ZW{fwd ? d.w : d.zw, g};
-    const View<double> ZUs{d.zu, g}, VIS{d.vis, g};
-    adj_viscosity(s, P, ZU, ZV, ZW, ZUs, VIS, S, f, k, j, i, sa, sb, sc);
+  if (!s.use_vd) {
+    if (fwd || !t.in) return;
+    atomicAdd(a.tg[F_ZU] + o, A);
+    atomicAdd(a.tg[F_ZV] + o, B);
+    atomicAdd(a.tg[F_ZW] + o, C);
+    return;
   }
-  adj_pw(s, P, U, V, W, S, k, j, i, sa, sb, sc);
+  __syncthreads();
+  VelCells c;
+  if (!fwd) {
+    c.u.add(0, 0, 0, A);
+    c.v.add(0, 0, 0, B);
+    c.w.add(0, 0, 0, C);
+  }
+  // viscosity_point's tau11p1 reads zu at x+1 also where the other stresses read u (the forward step)
+  const double zu_e = adj_viscosity(s, P, View<double>{fwd ? d.u : d.zu, g}, View<double>{fwd ? d.v : d.zv, g},
+                                    View<double>{fwd ? d.w : d.zw, g}, View<double>{d.zu, g}, View<double>{d.vis, g},
+                                    c, k, j, i, sa, sb, sc);
+  c.u.add(0, 0, 1, fwd ? 0.0 : zu_e);
+  if (fwd && t.in) atomicAdd(a.tg[F_ZU] + g.at(k, j, i + 1), zu_e);
+  constexpr int S1 = row_count(VD_U), S2 = S1 + row_count(VD_V), S3 = S2 + row_count(VD_W);
+  double *const tu = a.tg[fwd ? F_U : F_ZU], *const tv = a.tg[fwd ? F_V : F_ZV], *const tw = a.tg[fwd ? F_W : F_ZW];
+  RowSum ru[3], rv[3], rw[3], rn[3];
+  share_rows<VD_U, 0>(c.u, t, sh, ru);
+  share_rows<VD_V, S1>(c.v, t, sh, rv);
+  share_rows<VD_W, S2>(c.w, t, sh, rw);
+  share_rows<VD_VIS, S3>(c.vis, t, sh, rn);
+  __syncthreads();
+  add_rows<VD_U, 0>(tu, t, sh, ru);
+  add_rows<VD_V, S1>(tv, t, sh, rv);
+  add_rows<VD_W, S2>(tw, t, sh, rw);
+  add_rows<VD_VIS, S3>(a.tg[F_VIS], t, sh, rn);
 }
-
 
 // ---- scalar pass (eval_scalar: TVD advection of theta, diffusion, stepping) --------------------
 // derivatives of the limiter's building blocks as the forward evaluation branches them:
@@ -827,6 +896,9 @@ __device__ void adj_diffusion(const Scalars& s, const Prof<double>& P, const Vie
   S(F_DIFF, k - 1, j, i, dmb);
 }
 
+// 228 us at 128 x 128 x 96: bound by the dependent loads and divisions of the three faces at 16 warps an
+// SM, not by its atomics.  Row sums as in the momentum pass need 146 registers (8 warps: 451 us, 281 at
+// 128 registers with spills); one kernel for each face took 82, 90 and 99 us.
 __global__ void __launch_bounds__(128) k_hadj_scalar(Scalars s, Args a) {
   HADJ_POINT_INDEX
   const Geo g = geo(s);
@@ -882,155 +954,175 @@ __global__ void __launch_bounds__(128) k_hadj_scalar(Scalars s, Args a) {
 
 // ---- subgrid pass, levels 2 <= k <= nz-1 (smagorinsky_point, dry Richardson number) ------------
 // adjoint of half_squared_strain with the bar g of ssq
-__device__ void adj_strain(const Scalars& s, const Prof<double>& P, const View<double>& U, const View<double>& V,
-                           const View<double>& W, const Scatter& S, const VelAdj& f, int k, int j, int i,
-                           double g) {
+__device__ __forceinline__ void adj_strain(const Scalars& s, const Prof<double>& P, const View<double>& U, const View<double>& V,
+                           const View<double>& W, VelCells& A, int k, int j, int i, double g) {
   const double cx = s.cx, cy = s.cy, cx2 = s.cx2, cy2 = s.cy2;
   const double rdzn1 = P(P_RDZN, k + 1), rdzk = P(P_RDZ, k), rdzk1 = P(P_RDZ, k + 1);
   {  // ssq11
     const double b1 = g * cx2 * 2.0 * (U(k + 1, j, i) - U(k + 1, j, i - 1));
     const double b2 = g * cx2 * 2.0 * (U(k, j, i) - U(k, j, i - 1));
-    S(f.fu, k + 1, j, i, b1);
-    S(f.fu, k + 1, j, i - 1, -b1);
-    S(f.fu, k, j, i, b2);
-    S(f.fu, k, j, i - 1, -b2);
+    A.u.add(1, 0, 0, b1);
+    A.u.add(1, 0, -1, -b1);
+    A.u.add(0, 0, 0, b2);
+    A.u.add(0, 0, -1, -b2);
   }
   {  // ssq22
     const double b1 = g * cy2 * 2.0 * (V(k + 1, j, i) - V(k + 1, j - 1, i));
     const double b2 = g * cy2 * 2.0 * (V(k, j, i) - V(k, j - 1, i));
-    S(f.fv, k + 1, j, i, b1);
-    S(f.fv, k + 1, j - 1, i, -b1);
-    S(f.fv, k, j, i, b2);
-    S(f.fv, k, j - 1, i, -b2);
+    A.v.add(1, 0, 0, b1);
+    A.v.add(1, -1, 0, -b1);
+    A.v.add(0, 0, 0, b2);
+    A.v.add(0, -1, 0, -b2);
   }
   {  // ssq33
     const double b1 = g * 2.0 * ((W(k, j, i) - W(k - 1, j, i)) * rdzk) * rdzk;
     const double b2 = g * 2.0 * ((W(k + 1, j, i) - W(k, j, i)) * rdzk1) * rdzk1;
-    S(f.fw, k, j, i, b1 - b2);
-    S(f.fw, k - 1, j, i, -b1);
-    S(f.fw, k + 1, j, i, b2);
+    A.w.add(0, 0, 0, b1 - b2);
+    A.w.add(-1, 0, 0, -b1);
+    A.w.add(1, 0, 0, b2);
   }
   {  // ssq13
     const double x1 = (U(k + 1, j, i) - U(k, j, i)) * rdzn1 + (W(k, j, i + 1) - W(k, j, i)) * cx;
     const double x2 = (U(k + 1, j, i - 1) - U(k, j, i - 1)) * rdzn1 + (W(k, j, i) - W(k, j, i - 1)) * cx;
     const double b1 = g * x1, b2 = g * x2;
-    S(f.fu, k + 1, j, i, b1 * rdzn1);
-    S(f.fu, k, j, i, -b1 * rdzn1);
-    S(f.fw, k, j, i + 1, b1 * cx);
-    S(f.fw, k, j, i, (b2 - b1) * cx);
-    S(f.fu, k + 1, j, i - 1, b2 * rdzn1);
-    S(f.fu, k, j, i - 1, -b2 * rdzn1);
-    S(f.fw, k, j, i - 1, -b2 * cx);
+    A.u.add(1, 0, 0, b1 * rdzn1);
+    A.u.add(0, 0, 0, -b1 * rdzn1);
+    A.w.add(0, 0, 1, b1 * cx);
+    A.w.add(0, 0, 0, (b2 - b1) * cx);
+    A.u.add(1, 0, -1, b2 * rdzn1);
+    A.u.add(0, 0, -1, -b2 * rdzn1);
+    A.w.add(0, 0, -1, -b2 * cx);
   }
   {  // ssq23
     const double y1 = (W(k, j, i) - W(k, j - 1, i)) * cy + (V(k + 1, j - 1, i) - V(k, j - 1, i)) * rdzn1;
     const double y2 = (W(k, j + 1, i) - W(k, j, i)) * cy + (V(k + 1, j, i) - V(k, j, i)) * rdzn1;
     const double b1 = g * y1, b2 = g * y2;
-    S(f.fw, k, j, i, (b1 - b2) * cy);
-    S(f.fw, k, j - 1, i, -b1 * cy);
-    S(f.fv, k + 1, j - 1, i, b1 * rdzn1);
-    S(f.fv, k, j - 1, i, -b1 * rdzn1);
-    S(f.fw, k, j + 1, i, b2 * cy);
-    S(f.fv, k + 1, j, i, b2 * rdzn1);
-    S(f.fv, k, j, i, -b2 * rdzn1);
+    A.w.add(0, 0, 0, (b1 - b2) * cy);
+    A.w.add(0, -1, 0, -b1 * cy);
+    A.v.add(1, -1, 0, b1 * rdzn1);
+    A.v.add(0, -1, 0, -b1 * rdzn1);
+    A.w.add(0, 1, 0, b2 * cy);
+    A.v.add(1, 0, 0, b2 * rdzn1);
+    A.v.add(0, 0, 0, -b2 * rdzn1);
   }
-  for (int kk = k; kk <= k + 1; ++kk) {  // ssq12: four horizontal shears on levels k and k+1
+#pragma unroll
+  for (int dk = 0; dk <= 1; ++dk) {  // ssq12: four horizontal shears on levels k and k+1
+    const int kk = k + dk;
     const double z1 = (U(kk, j, i - 1) - U(kk, j - 1, i - 1)) * cy + (V(kk, j - 1, i) - V(kk, j - 1, i - 1)) * cx;
     const double z2 = (U(kk, j + 1, i - 1) - U(kk, j, i - 1)) * cy + (V(kk, j, i) - V(kk, j, i - 1)) * cx;
     const double z3 = (U(kk, j, i) - U(kk, j - 1, i)) * cy + (V(kk, j - 1, i + 1) - V(kk, j - 1, i)) * cx;
     const double z4 = (U(kk, j + 1, i) - U(kk, j, i)) * cy + (V(kk, j, i + 1) - V(kk, j, i)) * cx;
     const double b1 = 0.25 * g * z1, b2 = 0.25 * g * z2, b3 = 0.25 * g * z3, b4 = 0.25 * g * z4;
-    S(f.fu, kk, j, i - 1, (b1 - b2) * cy);
-    S(f.fu, kk, j - 1, i - 1, -b1 * cy);
-    S(f.fu, kk, j + 1, i - 1, b2 * cy);
-    S(f.fu, kk, j, i, (b3 - b4) * cy);
-    S(f.fu, kk, j - 1, i, -b3 * cy);
-    S(f.fu, kk, j + 1, i, b4 * cy);
-    S(f.fv, kk, j - 1, i, (b1 - b3) * cx);
-    S(f.fv, kk, j - 1, i - 1, -b1 * cx);
-    S(f.fv, kk, j, i, (b2 - b4) * cx);
-    S(f.fv, kk, j, i - 1, -b2 * cx);
-    S(f.fv, kk, j - 1, i + 1, b3 * cx);
-    S(f.fv, kk, j, i + 1, b4 * cx);
+    A.u.add(dk, 0, -1, (b1 - b2) * cy);
+    A.u.add(dk, -1, -1, -b1 * cy);
+    A.u.add(dk, 1, -1, b2 * cy);
+    A.u.add(dk, 0, 0, (b3 - b4) * cy);
+    A.u.add(dk, -1, 0, -b3 * cy);
+    A.u.add(dk, 1, 0, b4 * cy);
+    A.v.add(dk, -1, 0, (b1 - b3) * cx);
+    A.v.add(dk, -1, -1, -b1 * cx);
+    A.v.add(dk, 0, 0, (b2 - b4) * cx);
+    A.v.add(dk, 0, -1, -b2 * cx);
+    A.v.add(dk, -1, 1, b3 * cx);
+    A.v.add(dk, 0, 1, b4 * cx);
   }
 }
 
 // sum of v over the block (all of whose threads lie on one level), added to *dst by one thread
 __device__ __forceinline__ void block_add(double v, double* dst) {
-  __shared__ double part[4];
+  __shared__ double part[HY];
   for (int off = 16; off > 0; off >>= 1) v += __shfl_down_sync(0xffffffffu, v, off);
   const int lane = threadIdx.x & 31, warp = (threadIdx.y * blockDim.x + threadIdx.x) >> 5;
   if (lane == 0) part[warp] = v;
   __syncthreads();
   if (warp == 0 && lane == 0) {
-    const double t = (part[0] + part[1]) + (part[2] + part[3]);
+    double t = 0.0;
+    for (int q = 0; q < HY; ++q) t += part[q];
     if (t != 0.0) atomicAdd(dst, t);
   }
 }
 
-// one block of 32 x 4 threads per (x, y) tile of one level: the rneutml_sq adjoint of the level is
-// summed over the block before its single atomic (every point of a level adds to the same entry)
-__global__ void __launch_bounds__(128) k_hadj_smagorinsky(Scalars s, Args a) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  const int j = blockIdx.y * blockDim.y + threadIdx.y;
-  const int k = blockIdx.z + 1;
+// the cells half_squared_strain's adjoint adds to
+constexpr unsigned SS_U = cell(0, 0, -1) | cell(0, 0, 0) | cell(0, -1, -1) | cell(0, -1, 0) | cell(0, 1, -1) |
+                          cell(0, 1, 0) | cell(1, 0, -1) | cell(1, 0, 0) | cell(1, -1, -1) | cell(1, -1, 0) |
+                          cell(1, 1, -1) | cell(1, 1, 0);
+constexpr unsigned SS_V = xrow(0, 0) | xrow(0, -1) | xrow(1, 0) | xrow(1, -1);
+constexpr unsigned SS_W = xrow(0, 0) | cell(0, 1, 0) | cell(0, -1, 0) | cell(1, 0, 0) | cell(-1, 0, 0);
+
+// one block per (x, y) tile of one level: the rneutml_sq adjoint of the level is summed over the block
+// before its single atomic (every point of a level adds to the same entry)
+__global__ void __launch_bounds__(HX * HY) k_hadj_smagorinsky(Scalars s, Args a) {
+  constexpr int S1 = row_count(SS_U), S2 = S1 + row_count(SS_V);
+  __shared__ Rows<S2 + row_count(SS_W)> sh;
+  const Tile t(s);
+  const int k = t.k, j = min(t.j, s.ny - 1), i = min(t.i, s.nx - 1);
   if (k < 2 || k >= s.nz) return;  // uniform over the block
-  double prof_c = 0.0;
-  if (i < s.nx && j < s.ny) {
-    const long long o = (long long)(k - 1) * s.plane + (long long)j * s.nx + i;
-    const double vb = a.tg[F_VIS][o], db = a.tg[F_DIFF][o];
-    if (vb != 0.0 || db != 0.0) {
-      const Geo g = geo(s);
-      const Prof<double> P{s.prof, s.nz + 2};
-      const Scatter S{a.tg, g};
-      const DevState<double>& d = a.d;
-      const bool fwd = s.forward;
-      const View<double> U{fwd ? d.u : d.zu, g}, V{fwd ? d.v : d.zv, g}, W{fwd ? d.w : d.zw, g}, TH{d.th, g};
-      const VelAdj f = fwd ? VelAdj{F_U, F_V, F_W} : VelAdj{F_ZU, F_ZV, F_ZW};
-      // forward
-      const double ssq = half_squared_strain<double>(s, P, U, V, W, k, j, i);
-      double ri = 0.0;
-      if (!s.passive_th)
-        ri = (P(P_DTHREF, k) + TH(k + 1, j, i) - TH(k, j, i)) * P(P_RDZN, k + 1) * P(P_BUOY_CO, k) / ssq;
-      double vs = 0.0, df = 0.0, ri_vs = 0.0, ri_df = 0.0;  // stability functions and their ri-derivatives
-      if (ri <= 0.0) {
-        const double x1 = 1.0 - s.subc * ri, x2 = 1.0 - s.subb * ri;
-        vs = sqrt(x1);
-        const double r2 = sqrt(x2);
-        df = s.suba * r2;
-        ri_vs = vs > 0.0 ? -s.subc * 0.5 / vs : 0.0;
-        ri_df = r2 > 0.0 ? -s.subb * s.suba * 0.5 / r2 : 0.0;
-      } else if (ri > 0.0 && ri < s.ric) {
-        const double t1 = 1. - ri * s.ricinv;
-        const double t = t1 * t1;
-        const double rifac = t * t;
-        const double ev = 1. - s.subh * ri, ed = 1. - s.subg * ri;
-        vs = rifac * ev;
-        df = rifac * s.suba * ed;
-        const double rifac_ri = 2.0 * t * 2.0 * t1 * (-s.ricinv);
-        ri_vs = rifac_ri * ev - rifac * s.subh;
-        ri_df = rifac_ri * s.suba * ed - rifac * s.suba * s.subg;
-      }
-      const double rsq = P(P_RNEUTML_SQ, k), sq = sqrt(ssq);
-      const double sctmp = rsq * sq;
-      // reverse: vis = vs sctmp, diff = df sctmp, sctmp = rneutml_sq sqrt(ssq)
-      const double sct_b = vb * vs + db * df;
-      prof_c = sct_b * sq;
-      double ssq_b = sq > 0.0 ? sct_b * rsq * 0.5 / sq : 0.0;
-      const double ri_b = (vb * ri_vs + db * ri_df) * sctmp;
-      if (!s.passive_th && ri_b != 0.0) {
-        const double nb = ri_b * P(P_RDZN, k + 1) * P(P_BUOY_CO, k) / ssq;
-        S(F_TH, k + 1, j, i, nb);
-        S(F_TH, k, j, i, -nb);
-        ssq_b -= ri_b * ri / ssq;
-      }
-      adj_strain(s, P, U, V, W, S, f, k, j, i, ssq_b);
+  const Geo g = t.g;
+  const long long o = (long long)(k - 1) * s.plane + (long long)j * s.nx + i;
+  const Prof<double> P{s.prof, s.nz + 2};
+  const DevState<double>& d = a.d;
+  const bool fwd = s.forward;
+  const View<double> U{fwd ? d.u : d.zu, g}, V{fwd ? d.v : d.zv, g}, W{fwd ? d.w : d.zw, g}, TH{d.th, g};
+  const double vb = t.in ? a.tg[F_VIS][o] : 0.0, db = t.in ? a.tg[F_DIFF][o] : 0.0;
+  double prof_c = 0.0, ssq_b = 0.0;
+  if (vb != 0.0 || db != 0.0) {
+    // forward
+    const double ssq = half_squared_strain<double>(s, P, U, V, W, k, j, i);
+    double ri = 0.0;
+    if (!s.passive_th)
+      ri = (P(P_DTHREF, k) + TH(k + 1, j, i) - TH(k, j, i)) * P(P_RDZN, k + 1) * P(P_BUOY_CO, k) / ssq;
+    double vs = 0.0, df = 0.0, ri_vs = 0.0, ri_df = 0.0;  // stability functions and their ri-derivatives
+    if (ri <= 0.0) {
+      const double x1 = 1.0 - s.subc * ri, x2 = 1.0 - s.subb * ri;
+      vs = sqrt(x1);
+      const double r2 = sqrt(x2);
+      df = s.suba * r2;
+      ri_vs = vs > 0.0 ? -s.subc * 0.5 / vs : 0.0;
+      ri_df = r2 > 0.0 ? -s.subb * s.suba * 0.5 / r2 : 0.0;
+    } else if (ri > 0.0 && ri < s.ric) {
+      const double t1 = 1. - ri * s.ricinv;
+      const double t = t1 * t1;
+      const double rifac = t * t;
+      const double ev = 1. - s.subh * ri, ed = 1. - s.subg * ri;
+      vs = rifac * ev;
+      df = rifac * s.suba * ed;
+      const double rifac_ri = 2.0 * t * 2.0 * t1 * (-s.ricinv);
+      ri_vs = rifac_ri * ev - rifac * s.subh;
+      ri_df = rifac_ri * s.suba * ed - rifac * s.suba * s.subg;
+    }
+    const double rsq = P(P_RNEUTML_SQ, k), sq = sqrt(ssq);
+    const double sctmp = rsq * sq;
+    // reverse: vis = vs sctmp, diff = df sctmp, sctmp = rneutml_sq sqrt(ssq)
+    const double sct_b = vb * vs + db * df;
+    prof_c = sct_b * sq;
+    ssq_b = sq > 0.0 ? sct_b * rsq * 0.5 / sq : 0.0;
+    const double ri_b = (vb * ri_vs + db * ri_df) * sctmp;
+    if (!s.passive_th && ri_b != 0.0) {
+      const double nb = ri_b * P(P_RDZN, k + 1) * P(P_BUOY_CO, k) / ssq;
+      atomicAdd(a.tg[F_TH] + o + s.plane, nb);
+      atomicAdd(a.tg[F_TH] + o, -nb);
+      ssq_b -= ri_b * ri / ssq;
     }
   }
   block_add(prof_c, a.tg[F_PROF] + k);
+  VelCells c;
+  adj_strain(s, P, U, V, W, c, k, j, i, ssq_b);
+  double *const tu = a.tg[fwd ? F_U : F_ZU], *const tv = a.tg[fwd ? F_V : F_ZV], *const tw = a.tg[fwd ? F_W : F_ZW];
+  RowSum ru[3], rv[3], rw[3];
+  share_rows<SS_U, 0>(c.u, t, sh, ru);
+  share_rows<SS_V, S1>(c.v, t, sh, rv);
+  share_rows<SS_W, S2>(c.w, t, sh, rw);
+  __syncthreads();
+  add_rows<SS_U, 0>(tu, t, sh, ru);
+  add_rows<SS_V, S1>(tv, t, sh, rv);
+  add_rows<SS_W, S2>(tw, t, sh, rw);
 }
 }  // namespace hadj
 
+static dim3 row_grid(const Scalars& s) {
+  return dim3((s.nx + hadj::HX - 1) / hadj::HX, (s.ny + hadj::HY - 1) / hadj::HY, s.nz);
+}
+static dim3 row_block() { return dim3(hadj::HX, hadj::HY, 1); }
 static dim3 hadj_grid(const Scalars& s) { return dim3((s.nx + 31) / 32, (s.ny + 3) / 4, s.nz); }
 static dim3 hadj_block() { return dim3(32, 4, 1); }
 
@@ -1041,9 +1133,9 @@ bool hadj_pass(int pass, const Scalars& s, const DevState<double>& d, double* co
   for (int f = 0; f < F_COUNT; ++f) a.tg[f] = tg[f];
   for (int q = 0; q < 8; ++q) a.seed[q] = seed[q];
   switch (pass) {
-    case 1: hadj::k_hadj_momentum<<<hadj_grid(s), hadj_block(), 0, st>>>(s, a); return true;
+    case 1: hadj::k_hadj_momentum<<<row_grid(s), row_block(), 0, st>>>(s, a); return true;
     case 2: hadj::k_hadj_scalar<<<hadj_grid(s), hadj_block(), 0, st>>>(s, a); return true;
-    case 0: hadj::k_hadj_smagorinsky<<<hadj_grid(s), hadj_block(), 0, st>>>(s, a); return true;
+    case 0: hadj::k_hadj_smagorinsky<<<row_grid(s), row_block(), 0, st>>>(s, a); return true;
     case 3: hadj::k_hadj_pressure_source<<<hadj_grid(s), hadj_block(), 0, st>>>(s, a); return true;
     case 4: hadj::k_hadj_pstep_swap<<<hadj_grid(s), hadj_block(), 0, st>>>(s, a); return true;
     default: return false;

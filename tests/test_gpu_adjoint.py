@@ -292,3 +292,33 @@ def test_branch_flips_counts_differing_decisions(gpu_lib):
     assert a.branch_flips(b) > 0
     a.close()
     b.close()
+
+
+@pytest.mark.parametrize("nx,ny,nz", [(32, 8, 4), (36, 10, 5), (50, 18, 6), (6, 4, 24), (64, 10, 24)])
+@pytest.mark.parametrize("timestep,theta", [(1, True), (3, True), (3, False)])
+def test_adjoint_rows_of_ragged_tiles_match_tape(gpu_lib, nx, ny, nz, timestep, theta):
+    """The row sums of the hand-written adjoints, on whole and ragged tiles, a domain inside one
+    tile and every level next to the ground or the lid, against the tape; with a passive
+    theta too.  The bound is the one of the square grid above."""
+    st = ini.random_flow_state(nx, ny, nz, seed=8, amp_uv=1.0, amp_w=0.3, amp_th=0.5, ug=5.0)
+    res = []
+    for taped in (1, 0):
+        c = cf.dry_cbl_config(nx, ny, nz, DX, DZ, 1.0, ug=5.0, fcoriol=1e-4)
+        c.passive_th = 0 if theta else 1
+        c.adjoint_taped = taped
+        m = api.Model(c)
+        m.set_state({k: st[k] for k in STATE})
+        m.set_timestep(timestep)
+        for n, f in enumerate(STATE):
+            a = ini.uniform_noise((nz, ny, nx), 11, 50 + n, 1.0)
+            if f in ("w", "zw"):
+                a[0] = 0.0
+                a[-1] = 0.0
+            m.upload("adj:" + f, a)
+        rbar = m.adjoint_run(2, 2)
+        res.append(({f: m.download("adj:" + f) for f in STATE}, rbar))
+        m.close()
+    for f in STATE:
+        a, b = res[1][0][f], res[0][0][f]
+        assert np.abs(a - b).max() <= 1e-11 * np.abs(b).max(), f
+    assert abs(res[1][1] - res[0][1]) <= 1e-11 * abs(res[0][1])
