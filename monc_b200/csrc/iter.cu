@@ -201,25 +201,6 @@ __device__ void finish_refine(IterScalars* st, const double* s) {
   st->done = st->err < st->tol ? 1 : 0;
 }
 
-// (A x)(k, j, i) for 2 <= k <= nz (calc_Ax); x(o) gives the value at offset o.  The symmetric
-// form scales the horizontal part by A_vol(k).
-template <typename W, class X>
-__device__ __forceinline__ W apply_A_fn(const Geom& g, X x, int k, int j, int i) {
-  const int ie = i + 1 == g.nx ? 0 : i + 1, iw = i == 0 ? g.nx - 1 : i - 1;
-  const int jn = j + 1 == g.ny ? 0 : j + 1, js = j == 0 ? g.ny - 1 : j - 1;
-  const long long o = g.at(k, j, i);
-  const W xc = x(o);
-  W h = (W)g.A_n * (x(g.at(k, j, ie)) + x(g.at(k, j, iw))) + (W)g.A_e * (x(g.at(k, jn, i)) + x(g.at(k, js, i)));
-  if (g.symm) h = (W)g.avol(k) * h;
-  if (k == 2) return h + (W)g.au(k) * x(o + g.plane) + (W)g.ap(k) * xc;
-  if (k < g.nz) return h + (W)g.au(k) * x(o + g.plane) + (W)g.ad(k) * x(o - g.plane) + (W)g.ap(k) * xc;
-  return h + (W)g.ad(k) * x(o - g.plane) + (W)g.ap(k) * xc;
-}
-template <typename W>
-__device__ __forceinline__ W apply_A(const Geom& g, const W* __restrict__ x, int k, int j, int i) {
-  return apply_A_fn<W>(g, [&](long long o) { return x[o]; }, k, j, i);
-}
-
 __device__ __forceinline__ int block_id() { return blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z); }
 
 // The point kernels give each thread KZ consecutive levels of its column (blockIdx.z picks the
@@ -228,7 +209,62 @@ __device__ __forceinline__ int block_id() { return blockIdx.x + gridDim.x * (blo
 // dot-product kernels three times slower than their memory traffic.
 constexpr int KZ = 4;
 __device__ __forceinline__ int kz_lo() { return 2 + (int)blockIdx.z * KZ; }
-__device__ __forceinline__ int kz_hi(const Geom& g) { return min(g.nz, kz_lo() + KZ - 1); }
+
+// The operator's operand on a thread's KZ levels from k0 on and their neighbours: every load is issued
+// before the first value is used, 22 in flight a thread.  (Level by level, each level's loads waited for
+// the store of the level before: at 256 x 256 x 64 in FP64 the two products took 33.8 and
+// 39.6 us, now 33.0 and 36.4, the update 49.0, now 45.3.)
+template <typename W>
+struct ColumnStencil {
+  W c[KZ + 2], e[KZ], w[KZ], n[KZ], s[KZ];
+  template <class X>
+  __device__ __forceinline__ ColumnStencil(const Geom& g, X x, int k0, int j, int i) {
+    const int ie = i + 1 == g.nx ? 0 : i + 1, iw = i == 0 ? g.nx - 1 : i - 1;
+    const int jn = j + 1 == g.ny ? 0 : j + 1, js = j == 0 ? g.ny - 1 : j - 1;
+    const long long o = g.at(k0, j, i);
+    const long long oe = ie - i, ow = iw - i, on = (long long)(jn - j) * g.nx, os = (long long)(js - j) * g.nx;
+#pragma unroll
+    for (int q = 0; q < KZ + 2; ++q) {
+      const int k = k0 - 1 + q;
+      c[q] = k >= 2 && k <= g.nz ? x(o + (q - 1) * g.plane) : (W)0;
+    }
+#pragma unroll
+    for (int q = 0; q < KZ; ++q)
+      if (k0 + q <= g.nz) {
+        const long long oq = o + q * g.plane;
+        e[q] = x(oq + oe);
+        w[q] = x(oq + ow);
+        n[q] = x(oq + on);
+        s[q] = x(oq + os);
+      }
+  }
+  // (A x) at level k = k0 + q, 2 <= k <= nz (calc_Ax).  The symmetric form scales the horizontal part by
+  // A_vol(k).
+  __device__ __forceinline__ W apply(const Geom& g, int k, int q) const {
+    W h = (W)g.A_n * (e[q] + w[q]) + (W)g.A_e * (n[q] + s[q]);
+    if (g.symm) h = (W)g.avol(k) * h;
+    if (k == 2) return h + (W)g.au(k) * c[q + 2] + (W)g.ap(k) * c[q + 1];
+    if (k < g.nz) return h + (W)g.au(k) * c[q + 2] + (W)g.ad(k) * c[q] + (W)g.ap(k) * c[q + 1];
+    return h + (W)g.ad(k) * c[q] + (W)g.ap(k) * c[q + 1];
+  }
+};
+// another array on the KZ levels
+template <typename W, class X>
+__device__ __forceinline__ void load_levels(const Geom& g, X x, int k0, int j, int i, W (&v)[KZ]) {
+  const long long o = g.at(k0, j, i);
+#pragma unroll
+  for (int q = 0; q < KZ; ++q)
+    if (k0 + q <= g.nz) v[q] = x[o + q * g.plane];
+}
+// f(q, k, offset) for the thread's levels
+template <class F>
+__device__ __forceinline__ void each_level(const Geom& g, int k0, int j, int i, F f) {
+  const long long o = g.at(k0, j, i);
+#pragma unroll
+  for (int q = 0; q < KZ; ++q)
+    if (k0 + q <= g.nz) f(q, k0 + q, o + q * g.plane);
+}
+
 
 // r = b - A x, cr = r; sums <r, r> and <b, b>; initial scalars
 template <typename W>
@@ -236,66 +272,99 @@ __global__ void __launch_bounds__(NTH) k_bicg_init(Geom g, const W* __restrict__
                                                     double* partials, int nblocks, IterScalars* st, double sc_floor) {
   const int i = blockIdx.x * BX + threadIdx.x, j = g.j0 + blockIdx.y * BY + threadIdx.y;
   double v[2] = {0.0, 0.0};
-  if (i < g.nx && j < g.j1)
-    for (int k = kz_lo(); k <= kz_hi(g); ++k) {
-      const long long o = g.at(k, j, i);
-      const W rv = b[o] - apply_A<W>(g, x, k, j, i);
+  if (i < g.nx && j < g.j1) {
+    const int k0 = kz_lo();
+    const ColumnStencil<W> A(g, [&](long long o) { return x[o]; }, k0, j, i);
+    W bv[KZ];
+    load_levels(g, b, k0, j, i, bv);
+    each_level(g, k0, j, i, [&](int q, int k, long long o) {
+      const W rv = bv[q] - A.apply(g, k, q);
       r[o] = rv;
       cr[o] = rv;
       v[0] += (double)rv * (double)rv;
-      v[1] += (double)b[o] * (double)b[o];
-    }
+      v[1] += (double)bv[q] * (double)bv[q];
+    });
+  }
   block_partials<2>(v, partials, nblocks, block_id());
   double s[2];
   if (last_block_sums<2>(st, partials, nblocks, s)) finish_init(st, s, sc_floor);
 }
 
 // column LU solve of the vertical operator: out = M^-1 in (precond); `tmp` holds the forward sweep.
-// A thread walks its column level by level; CH levels of its input are loaded before the first of
-// them is used, so that the loads are in flight together instead of one round trip per level
-// (one thread per column leaves too few warps to hide the latency otherwise).
+// A thread walks its column level by level; the operands of CH levels are loaded while the CH levels
+// before them are worked on, so that a round trip to memory is paid once and not once a level or chunk
+// (one thread per column leaves too few warps to hide it otherwise).  256 x 256 x 64 in FP64: the two
+// column kernels of an iteration took 57.8 and 54.2 us with loads a chunk at a time, 27.1 and 26.3 so.
+// ld(o) loads a level's operands, val(o, raw) gives its input.
 constexpr int CH = 8;
-template <typename W, class In>
-__device__ __forceinline__ void column_precond(const Geom& g, In in, W* tmp, int j, int i) {
+template <typename W, class Raw, class Ld, class Val>
+__device__ __forceinline__ void column_precond(const Geom& g, Ld ld, Val val, W* tmp, int j, int i) {
   long long o = g.at(2, j, i);
-  W sp = in(o) * (W)g.lud(2);
+  const Raw first = ld(o);
+  Raw next[CH];
+#pragma unroll
+  for (int q = 0; q < CH; ++q)
+    if (3 + q <= g.nz) next[q] = ld(o + (long long)(q + 1) * g.plane);
+  W sp = val(o, first) * (W)g.lud(2);
   tmp[o] = sp;
   for (int k0 = 3; k0 <= g.nz; k0 += CH) {
-    W x[CH];
+    Raw x[CH];
+#pragma unroll
+    for (int q = 0; q < CH; ++q) x[q] = next[q];
 #pragma unroll
     for (int q = 0; q < CH; ++q)
-      if (k0 + q <= g.nz) x[q] = in(o + (long long)(q + 1) * g.plane);
+      if (k0 + CH + q <= g.nz) next[q] = ld(o + (long long)(CH + q + 1) * g.plane);
 #pragma unroll
     for (int q = 0; q < CH; ++q)
       if (k0 + q <= g.nz) {
         o += g.plane;
-        sp = (x[q] - (W)g.ad(k0 + q) * sp) * (W)g.lud(k0 + q);
+        sp = (val(o, x[q]) - (W)g.ad(k0 + q) * sp) * (W)g.lud(k0 + q);
         tmp[o] = sp;
       }
   }
 }
 
-// back substitution sk(k) = tmp(k) - luu(k) sk(k+1) from the top level down to level 2;
-// out(o, sk) receives each level's value
-template <typename W, class Out>
-__device__ __forceinline__ void column_back(const Geom& g, const W* tmp, int j, int i, Out out) {
+// back substitution sk(k) = tmp(k) - luu(k) sk(k+1) from the top level down to level 2; out(o, sk, raw)
+// receives each level's value and what ld(o) loaded for it
+template <typename W, class Raw, class Ld, class Out>
+__device__ __forceinline__ void column_back(const Geom& g, const W* tmp, int j, int i, Ld ld, Out out) {
   long long o = g.at(g.nz, j, i);
   W sk = tmp[o];
-  out(o, sk);
+  const Raw first = ld(o);
+  W tn[CH];
+  Raw next[CH];
+#pragma unroll
+  for (int q = 0; q < CH; ++q)
+    if (g.nz - 1 - q >= 2) {
+      tn[q] = tmp[o - (long long)(q + 1) * g.plane];
+      next[q] = ld(o - (long long)(q + 1) * g.plane);
+    }
+  out(o, sk, first);
   for (int k0 = g.nz - 1; k0 >= 2; k0 -= CH) {
     W t[CH];
+    Raw x[CH];
+#pragma unroll
+    for (int q = 0; q < CH; ++q) t[q] = tn[q], x[q] = next[q];
 #pragma unroll
     for (int q = 0; q < CH; ++q)
-      if (k0 - q >= 2) t[q] = tmp[o - (long long)(q + 1) * g.plane];
+      if (k0 - CH - q >= 2) {
+        tn[q] = tmp[o - (long long)(CH + q + 1) * g.plane];
+        next[q] = ld(o - (long long)(CH + q + 1) * g.plane);
+      }
 #pragma unroll
     for (int q = 0; q < CH; ++q)
       if (k0 - q >= 2) {
         o -= g.plane;
         sk = t[q] - (W)g.luu(k0 - q) * sk;
-        out(o, sk);
+        out(o, sk, x[q]);
       }
   }
 }
+struct NoRaw {};
+template <typename W>
+struct TwoRaw {
+  W a, b;
+};
 
 // iteration step 1: search direction pp
 template <typename W>
@@ -307,10 +376,14 @@ __global__ void __launch_bounds__(NTH) k_bicg_direction(Geom g, const W* __restr
   const bool first = st->it == 1;
   const double bet_d = (st->rho / st->rho_prev) * (st->alf / st->omg);
   const W bet = (W)bet_d, bo = (W)(bet_d * st->omg);
-  if (first) column_precond<W>(g, [&](long long o) { return r[o]; }, tmp, j, i);
-  else column_precond<W>(g, [&](long long o) { return r[o] - bo * v[o]; }, tmp, j, i);
+  if (first)
+    column_precond<W, W>(g, [&](long long o) { return r[o]; }, [&](long long, W x) { return x; }, tmp, j, i);
+  else
+    column_precond<W, TwoRaw<W>>(g, [&](long long o) { return TwoRaw<W>{r[o], v[o]}; },
+                                 [&](long long, const TwoRaw<W>& x) { return x.a - bo * x.b; }, tmp, j, i);
   // back substitution, then pp = s + bet*pp
-  column_back<W>(g, tmp, j, i, [&](long long o, W sk) { pp[o] = first ? sk : sk + bet * pp[o]; });
+  column_back<W, W>(g, tmp, j, i, [&](long long o) { return pp[o]; },
+                    [&](long long o, W sk, W old) { pp[o] = first ? sk : sk + bet * old; });
 }
 
 // iteration step 2: v = A pp, alf = rho / <cr, v>
@@ -320,13 +393,17 @@ __global__ void __launch_bounds__(NTH) k_bicg_apply_dot(Geom g, const W* __restr
   if (st->done) return;
   const int i = blockIdx.x * BX + threadIdx.x, j = g.j0 + blockIdx.y * BY + threadIdx.y;
   double a[1] = {0.0};
-  if (i < g.nx && j < g.j1)
-    for (int k = kz_lo(); k <= kz_hi(g); ++k) {
-      const long long o = g.at(k, j, i);
-      const W vv = apply_A<W>(g, pp, k, j, i);
+  if (i < g.nx && j < g.j1) {
+    const int k0 = kz_lo();
+    const ColumnStencil<W> A(g, [&](long long o) { return pp[o]; }, k0, j, i);
+    W c[KZ];
+    load_levels(g, cr, k0, j, i, c);
+    each_level(g, k0, j, i, [&](int q, int k, long long o) {
+      const W vv = A.apply(g, k, q);
       v[o] = vv;
-      a[0] += (double)cr[o] * (double)vv;
-    }
+      a[0] += (double)c[q] * (double)vv;
+    });
+  }
   block_partials<1>(a, partials, nblocks, block_id());
   double s[1];
   if (last_block_sums<1>(st, partials, nblocks, s)) finish_apply_dot(st, s);
@@ -340,12 +417,14 @@ __global__ void __launch_bounds__(NTH) k_bicg_half_step(Geom g, const W* __restr
   const int i = blockIdx.x * BX + threadIdx.x, j = g.j0 + blockIdx.y * BY + threadIdx.y;
   if (i >= g.nx || j >= g.j1) return;
   const W alf = (W)st->alf;
-  column_precond<W>(g, [&](long long o) {
-    const W sv = r[o] - alf * v[o];
-    s_[o] = sv;
-    return sv;
-  }, tmp, j, i);
-  column_back<W>(g, tmp, j, i, [&](long long o, W ck) { cs[o] = ck; });
+  column_precond<W, TwoRaw<W>>(g, [&](long long o) { return TwoRaw<W>{r[o], v[o]}; },
+                               [&](long long o, const TwoRaw<W>& x) {
+                                 const W sv = x.a - alf * x.b;
+                                 s_[o] = sv;
+                                 return sv;
+                               },
+                               tmp, j, i);
+  column_back<W, NoRaw>(g, tmp, j, i, [&](long long) { return NoRaw{}; }, [&](long long o, W ck, NoRaw) { cs[o] = ck; });
 }
 
 // iteration step 4: t = A cs; tt, ts, ss; omg, err
@@ -355,16 +434,20 @@ __global__ void __launch_bounds__(NTH) k_bicg_apply_dots(Geom g, const W* __rest
   if (st->done) return;
   const int i = blockIdx.x * BX + threadIdx.x, j = g.j0 + blockIdx.y * BY + threadIdx.y;
   double a[3] = {0.0, 0.0, 0.0};
-  if (i < g.nx && j < g.j1)
-    for (int k = kz_lo(); k <= kz_hi(g); ++k) {
-      const long long o = g.at(k, j, i);
-      const W tv = apply_A<W>(g, cs, k, j, i);
+  if (i < g.nx && j < g.j1) {
+    const int k0 = kz_lo();
+    const ColumnStencil<W> A(g, [&](long long o) { return cs[o]; }, k0, j, i);
+    W sv[KZ];
+    load_levels(g, s_, k0, j, i, sv);
+    each_level(g, k0, j, i, [&](int q, int k, long long o) {
+      const W tv = A.apply(g, k, q);
       t[o] = tv;
-      const double td = (double)tv, sd = (double)s_[o];
+      const double td = (double)tv, sd = (double)sv[q];
       a[0] += td * td;
       a[1] += td * sd;
       a[2] += sd * sd;
-    }
+    });
+  }
   block_partials<3>(a, partials, nblocks, block_id());
   double s[3];
   if (last_block_sums<3>(st, partials, nblocks, s)) finish_apply_dots(st, s);
@@ -381,13 +464,20 @@ __global__ void __launch_bounds__(NTH) k_bicg_update(Geom g, W* x, const W* __re
   double a[1] = {0.0};
   if (i < g.nx && j < g.j1) {
     const W alf = (W)st->alf, omg = (W)st->omg;
-    for (int k = kz_lo(); k <= kz_hi(g); ++k) {
-      const long long o = g.at(k, j, i);
-      x[o] = x[o] + alf * pp[o] + omg * cs[o];
-      const W rv = s_[o] - omg * t[o];
+    const int k0 = kz_lo();
+    W xv[KZ], pv[KZ], cv[KZ], sv[KZ], tv[KZ], rc[KZ];
+    load_levels(g, x, k0, j, i, xv);
+    load_levels(g, pp, k0, j, i, pv);
+    load_levels(g, cs, k0, j, i, cv);
+    load_levels(g, s_, k0, j, i, sv);
+    load_levels(g, t, k0, j, i, tv);
+    load_levels(g, cr, k0, j, i, rc);
+    each_level(g, k0, j, i, [&](int q, int, long long o) {
+      x[o] = xv[q] + alf * pv[q] + omg * cv[q];
+      const W rv = sv[q] - omg * tv[q];
       r[o] = rv;
-      a[0] += (double)rv * (double)cr[o];
-    }
+      a[0] += (double)rv * (double)rc[q];
+    });
   }
   block_partials<1>(a, partials, nblocks, block_id());
   double s[1];
@@ -426,15 +516,19 @@ __global__ void __launch_bounds__(NTH) k_cg_init(Geom g, const W* __restrict__ x
                                                   int scale_rhs) {
   const int i = blockIdx.x * BX + threadIdx.x, j = g.j0 + blockIdx.y * BY + threadIdx.y;
   double v[2] = {0.0, 0.0};
-  if (i < g.nx && j < g.j1)
-    for (int k = kz_lo(); k <= kz_hi(g); ++k) {
-      const long long o = g.at(k, j, i);
-      const W bv = scale_rhs ? b[o] * (W)g.avol(k) : b[o];
-      const W rv = bv - apply_A<W>(g, x, k, j, i);
+  if (i < g.nx && j < g.j1) {
+    const int k0 = kz_lo();
+    const ColumnStencil<W> A(g, [&](long long o) { return x[o]; }, k0, j, i);
+    W bl[KZ];
+    load_levels(g, b, k0, j, i, bl);
+    each_level(g, k0, j, i, [&](int q, int k, long long o) {
+      const W bv = scale_rhs ? bl[q] * (W)g.avol(k) : bl[q];
+      const W rv = bv - A.apply(g, k, q);
       r[o] = rv;
       v[0] += (double)bv * (double)bv;
       v[1] += (double)rv * (double)rv;
-    }
+    });
+  }
   block_partials<2>(v, partials, nblocks, block_id());
   double s[2];
   if (last_block_sums<2>(st, partials, nblocks, s)) finish_cg_init(st, s, sc_floor);
@@ -448,10 +542,10 @@ __global__ void __launch_bounds__(NTH) k_cg_precond(Geom g, const W* __restrict_
   const int i = blockIdx.x * BX + threadIdx.x, j = g.j0 + blockIdx.y * BY + threadIdx.y;
   double a[1] = {0.0};
   if (i < g.nx && j < g.j1) {
-    column_precond<W>(g, [&](long long o) { return r[o]; }, tmp, j, i);
-    column_back<W>(g, tmp, j, i, [&](long long o, W zk) {
+    column_precond<W, W>(g, [&](long long o) { return r[o]; }, [&](long long, W x) { return x; }, tmp, j, i);
+    column_back<W, W>(g, tmp, j, i, [&](long long o) { return r[o]; }, [&](long long o, W zk, W rv) {
       z[o] = zk;
-      a[0] += (double)zk * (double)r[o];
+      a[0] += (double)zk * (double)rv;
     });
   }
   block_partials<1>(a, partials, nblocks, block_id());
@@ -476,15 +570,17 @@ __global__ void __launch_bounds__(NTH) k_cg_apply(Geom g, const W* __restrict__ 
   const W bet = (W)st->bet;
   auto pn = [&](long long o) { return first ? z[o] : axpy_rn<W>(bet, p_old[o], z[o]); };
   double a[1] = {0.0};
-  if (i < g.nx && j < g.j1)
-    for (int k = kz_lo(); k <= kz_hi(g); ++k) {
-      const long long o = g.at(k, j, i);
-      const W pc = pn(o);
+  if (i < g.nx && j < g.j1) {
+    const int k0 = kz_lo();
+    const ColumnStencil<W> A(g, pn, k0, j, i);
+    each_level(g, k0, j, i, [&](int q, int k, long long o) {
+      const W pc = A.c[q + 1];
       p_new[o] = pc;
-      const W av = apply_A_fn<W>(g, pn, k, j, i);
+      const W av = A.apply(g, k, q);
       Ax[o] = av;
       a[0] += (double)pc * (double)av;
-    }
+    });
+  }
   block_partials<1>(a, partials, nblocks, block_id());
   double s[1];
   if (last_block_sums<1>(st, partials, nblocks, s)) finish_cg_apply(st, s);
@@ -499,13 +595,18 @@ __global__ void __launch_bounds__(NTH) k_cg_update(Geom g, W* x, const W* __rest
   double a[1] = {0.0};
   if (i < g.nx && j < g.j1) {
     const W alf = (W)st->alf;
-    for (int k = kz_lo(); k <= kz_hi(g); ++k) {
-      const long long o = g.at(k, j, i);
-      x[o] = x[o] + alf * p[o];
-      const W rv = r[o] - alf * Ax[o];
+    const int k0 = kz_lo();
+    W xv[KZ], pv[KZ], rl[KZ], av[KZ];
+    load_levels(g, x, k0, j, i, xv);
+    load_levels(g, p, k0, j, i, pv);
+    load_levels(g, r, k0, j, i, rl);
+    load_levels(g, Ax, k0, j, i, av);
+    each_level(g, k0, j, i, [&](int q, int, long long o) {
+      x[o] = xv[q] + alf * pv[q];
+      const W rv = rl[q] - alf * av[q];
       r[o] = rv;
       a[0] += (double)rv * (double)rv;
-    }
+    });
   }
   block_partials<1>(a, partials, nblocks, block_id());
   double s[1];
@@ -518,16 +619,20 @@ __global__ void __launch_bounds__(NTH) k_refine_residual(Geom g, const double* _
                                                           IterScalars* st) {
   const int i = blockIdx.x * BX + threadIdx.x, j = g.j0 + blockIdx.y * BY + threadIdx.y;
   double v[2] = {0.0, 0.0};
-  if (i < g.nx && j < g.j1)
-    for (int k = kz_lo(); k <= kz_hi(g); ++k) {
-      const long long o = g.at(k, j, i);
-      const double bv = g.symm ? b[o] * g.avol(k) : b[o];
-      const double rv = bv - apply_A<double>(g, x, k, j, i);
+  if (i < g.nx && j < g.j1) {
+    const int k0 = kz_lo();
+    const ColumnStencil<double> A(g, [&](long long o) { return x[o]; }, k0, j, i);
+    double bl[KZ];
+    load_levels(g, b, k0, j, i, bl);
+    each_level(g, k0, j, i, [&](int q, int k, long long o) {
+      const double bv = g.symm ? bl[q] * g.avol(k) : bl[q];
+      const double rv = bv - A.apply(g, k, q);
       r[o] = rv;
       r32[o] = (float)rv;
       v[0] += rv * rv;
       v[1] += bv * bv;
-    }
+    });
+  }
   block_partials<2>(v, partials, nblocks, block_id());
   double s[2];
   if (last_block_sums<2>(st, partials, nblocks, s)) finish_refine(st, s);
@@ -541,7 +646,7 @@ __global__ void __launch_bounds__(NTH) k_compat_sum(Geom g, const double* __rest
   const int i = blockIdx.x * BX + threadIdx.x, j = g.j0 + blockIdx.y * BY + threadIdx.y;
   double v[1] = {0.0};
   if (i < g.nx && j < g.j1)
-    for (int k = kz_lo(); k <= kz_hi(g); ++k) v[0] += g.vol(k) * b[g.at(k, j, i)];
+    each_level(g, kz_lo(), j, i, [&](int, int k, long long o) { v[0] += g.vol(k) * b[o]; });
   block_partials<1>(v, partials, nblocks, block_id());
   double s[1];
   if (last_block_sums<1>(st, partials, nblocks, s)) finish_compat(st, s, g);
