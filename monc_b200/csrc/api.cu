@@ -921,7 +921,7 @@ static int adjoint_run(mgpu_handle* h, int nsteps, int interval, double* rmlmax_
   const size_t n = field_elems(h);
   const int t0 = h->timestep;
   const int nck = (nsteps + interval - 1) / interval;
-  while ((int)a->ckpt.size() < 8 * nck) {
+  while ((int)a->ckpt.size() < 8 * (nck - 1)) {  // the last segment needs none
     double* p = nullptr;
     if (ad_alloc(h, &p, n)) return MGPU_ERR_CUDA;
     a->ckpt.push_back(p);
