@@ -11,13 +11,14 @@
 //    through the face below) is carried up in registers;
 //  * the reference density cancels (Boussinesq: rho = rhon on every level);
 //  * the buoyancy of a level is formed once, from the q fields that have a weight, loaded a whole
-//    level before it is used (used at once, those loads held the warps up: 0.282 against 0.254 ms).
-// 256 x 256 x 128: FP64 0.275 -> 0.254 ms (738 MB, 0.113 ms), FP32 0.170 -> 0.156 ms; moist
-// 512 x 512 x 160: 1.78 -> 1.17 and 1.02 -> 0.74 ms; 1024 x 1024 x 200 with five q fields, FP32:
-// 7.07 -> 3.61 ms.  What is left is latency with 16 warps per SM (128 registers, 90 KB): copies in
-// flight, shared-memory loads and two barriers a level; issue slots 40% used.
+//    level before it is used (used at once, those loads held the warps up: 0.282 against 0.254 ms
+//    with two barriers a level).
+// 256 x 256 x 128: FP64 0.275 -> 0.246 ms (738 MB, 0.113 ms), FP32 0.170 -> 0.151 ms; moist
+// 512 x 512 x 160: 1.78 -> 1.15 and 1.02 -> 0.71 ms; 1024 x 1024 x 200 with five q fields, FP32:
+// 7.07 -> 3.40 ms.  What is left is latency with 16 warps per SM (128 registers, 90 KB): copies in
+// flight, shared-memory loads and a barrier a level.
 // Sizes that no tile divides run here too: 360 x 300 x 81 in FP64 took 1.67 ms in the point kernel
-// for momentum and theta, now 0.29 and 0.33 ms.
+// for momentum and theta, now 0.28 and 0.28 ms.
 #pragma once
 
 namespace mgpu {
