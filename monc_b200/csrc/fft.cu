@@ -1580,7 +1580,7 @@ template void slab_solve_columns<double>(const FftPlanDev&, const Scalars&, void
 template void slab_solve_columns<float>(const FftPlanDev&, const Scalars&, void*, int, int, int, bool, cudaStream_t,
                                         int64_t*);
 
-// ---- horizontal-mean diagnostics: one block per level, FP64 accumulation in a fixed order ----
+// ---- horizontal-mean diagnostics: one cluster of blocks per level, FP64 accumulation in a fixed order ----
 // Level sums split over a cluster of PSPLIT blocks (one cluster per level): block r sums its
 // contiguous share of the level's points, each thread in a fixed stride order and the block by a
 // tree; block 0 then adds the PSPLIT partial sums in rank order through distributed shared memory.
