@@ -942,6 +942,7 @@ static int adjoint_run(mgpu_handle* h, int nsteps, int interval, double* rmlmax_
     int rc = step_once<double>(h, d);
     if (rc) return rc;
   }
+  const double t_end = h->time;  // the recomputed steps move the clock on
   if (nck > 1) {  // recomputing the earlier segments overwrites the state
     state_ptrs(d, X);
     copy_state(h, a->final_state, X);
@@ -975,6 +976,7 @@ static int adjoint_run(mgpu_handle* h, int nsteps, int interval, double* rmlmax_
     copy_state(h, X, a->final_state);
   }
   h->timestep = t0 + nsteps;
+  h->time = t_end;
   int ovf = 0;
   std::vector<double> pb(h->cfg.nz + 2);
   CK(cudaMemcpyAsync(&ovf, a->overflow, sizeof(int), cudaMemcpyDeviceToHost, h->stream));

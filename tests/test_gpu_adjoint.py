@@ -322,3 +322,21 @@ def test_adjoint_rows_of_ragged_tiles_match_tape(gpu_lib, nx, ny, nz, timestep, 
         a, b = res[1][0][f], res[0][0][f]
         assert np.abs(a - b).max() <= 1e-11 * np.abs(b).max(), f
     assert abs(res[1][1] - res[0][1]) <= 1e-11 * abs(res[0][1])
+
+
+@pytest.mark.parametrize("nsteps,interval", [(1, 1), (4, 4), (5, 2), (6, 1)])
+def test_adjoint_run_leaves_the_clock_of_its_forward_steps(gpu_lib, nsteps, interval):
+    """The model stands after nsteps steps, whatever the reverse sweep recomputed: its timestep and time are
+    those of a model that took the steps."""
+    metas = []
+    for adjoint in (False, True):
+        m = api.Model(cf.dry_cbl_config(32, 8, 6, DX, DZ, 0.25, ug=5.0))
+        m.set_timestep(3)
+        if adjoint:
+            m.adjoint_run(nsteps, interval)
+        else:
+            m.step(nsteps)
+        metas.append(m.checkpoint_state())
+        m.close()
+    assert metas[1].timestep == metas[0].timestep
+    assert metas[1].time == metas[0].time
