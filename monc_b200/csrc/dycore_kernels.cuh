@@ -21,6 +21,7 @@
 
 #include "dycore.h"
 #include "dycore_device.cuh"
+#include "launch_limits.h"
 
 #ifndef KVARIANT
 #define KVARIANT exact
@@ -1756,17 +1757,11 @@ static inline int choose_level_chunks(int tiles, int slots, int levels, double p
 
 // the TVD advection of flow component DIM on the centred step, into src (one launch)
 template <typename T, int DIM>
-static int launch_flow_tvd(const Scalars& s, DevState<T>& d, T* src, int tiles, int nsm, int levels,
-                           cudaStream_t st) {
+static int launch_flow_tvd(const Scalars& s, DevState<T>& d, T* src, int tiles, int levels, cudaStream_t st) {
   const size_t smem = tiled::flow_smem<T, DIM>();
-  static int occ = 0;
-  if (!occ) {
-    cudaFuncSetAttribute(k_f_flow_tvd_tiled<T, DIM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    cudaFuncSetAttribute(k_f_flow_tvd_tiled<T, DIM>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_f_flow_tvd_tiled<T, DIM>, tiled::NT, smem);
-    if (occ < 1) occ = 1;
-  }
-  const int nc = s.level_chunks > 0 ? s.level_chunks : choose_level_chunks(tiles, occ * nsm, levels);
+  static LaunchTable table;
+  const LaunchLimits lim = launch_limits(table, {(const void*)k_f_flow_tvd_tiled<T, DIM>}, tiled::NT, smem);
+  const int nc = s.level_chunks > 0 ? s.level_chunks : choose_level_chunks(tiles, lim.occ * lim.nsm, levels);
   const int kc = (levels + nc - 1) / nc;
   dim3 grid(s.nx / tiled::TX, s.ny / tiled::TY, (levels + kc - 1) / kc);
   k_f_flow_tvd_tiled<T, DIM><<<grid, dim3(tiled::TX, tiled::TY, 1), smem, st>>>(s, d, kc, src);
@@ -1775,16 +1770,11 @@ static int launch_flow_tvd(const Scalars& s, DevState<T>& d, T* src, int tiles, 
 
 // the moist scalar step of theta and two q fields (one launch)
 template <typename T>
-static int launch_moist(const Scalars& s, DevState<T>& d, int tiles, int nsm, int levels, cudaStream_t st) {
+static int launch_moist(const Scalars& s, DevState<T>& d, int tiles, int levels, cudaStream_t st) {
   const size_t smem = tiled::moist_smem<T>();
-  static int occ = 0;
-  if (!occ) {
-    cudaFuncSetAttribute(k_f_moist_tiled<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    cudaFuncSetAttribute(k_f_moist_tiled<T>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_f_moist_tiled<T>, tiled::NT, smem);
-    if (occ < 1) occ = 1;
-  }
-  const int nc = s.level_chunks > 0 ? s.level_chunks : choose_level_chunks(tiles, occ * nsm, levels);
+  static LaunchTable table;
+  const LaunchLimits lim = launch_limits(table, {(const void*)k_f_moist_tiled<T>}, tiled::NT, smem);
+  const int nc = s.level_chunks > 0 ? s.level_chunks : choose_level_chunks(tiles, lim.occ * lim.nsm, levels);
   const int kc = (levels + nc - 1) / nc;
   dim3 grid(s.nx / tiled::TX, s.ny / tiled::TY, (levels + kc - 1) / kc);
   k_f_moist_tiled<T><<<grid, dim3(tiled::TX, tiled::TY, 1), smem, st>>>(s, d, kc);
@@ -1795,17 +1785,12 @@ static int launch_moist(const Scalars& s, DevState<T>& d, int tiles, int nsm, in
 // cloud and stepping included), or one launch per scalar writing its source, then saturation
 // adjustment and stepping
 template <typename T>
-static int launch_scalar_part(const Scalars& s, DevState<T>& d, int tiles, int nsm, int levels, cudaStream_t st) {
-  if (s.nq == 2) return launch_moist<T>(s, d, tiles, nsm, levels, st);
+static int launch_scalar_part(const Scalars& s, DevState<T>& d, int tiles, int levels, cudaStream_t st) {
+  if (s.nq == 2) return launch_moist<T>(s, d, tiles, levels, st);
   const size_t sm_s = tiled::scalar_smem<T>();
-  static int occ_s = 0;
-  if (!occ_s) {
-    cudaFuncSetAttribute(k_f_scalar_tiled<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_s);
-    cudaFuncSetAttribute(k_f_scalar_tiled<T>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_s, k_f_scalar_tiled<T>, tiled::NT, sm_s);
-    if (occ_s < 1) occ_s = 1;
-  }
-  const int nc_s = s.level_chunks > 0 ? s.level_chunks : choose_level_chunks(tiles, occ_s * nsm, levels, 0.002);
+  static LaunchTable table;
+  const LaunchLimits lim = launch_limits(table, {(const void*)k_f_scalar_tiled<T>}, tiled::NT, sm_s);
+  const int nc_s = s.level_chunks > 0 ? s.level_chunks : choose_level_chunks(tiles, lim.occ * lim.nsm, levels, 0.002);
   const int kc_s = (levels + nc_s - 1) / nc_s;
   dim3 block(tiled::TX, tiled::TY, 1);
   dim3 grid_s(s.nx / tiled::TX, s.ny / tiled::TY, (levels + kc_s - 1) / kc_s);
@@ -1820,10 +1805,9 @@ static int launch_scalar_part(const Scalars& s, DevState<T>& d, int tiles, int n
   return s.nq + 2;
 }
 template <typename T>
-static int launch_flow_part(const Scalars& s, DevState<T>& d, int tiles, int nsm, int levels, cudaStream_t st) {
-  return launch_flow_tvd<T, 0>(s, d, d.su, tiles, nsm, levels, st) +
-         launch_flow_tvd<T, 1>(s, d, d.sv, tiles, nsm, levels, st) +
-         launch_flow_tvd<T, 2>(s, d, d.sw, tiles, nsm, levels, st);
+static int launch_flow_part(const Scalars& s, DevState<T>& d, int tiles, int levels, cudaStream_t st) {
+  return launch_flow_tvd<T, 0>(s, d, d.su, tiles, levels, st) + launch_flow_tvd<T, 1>(s, d, d.sv, tiles, levels, st) +
+         launch_flow_tvd<T, 2>(s, d, d.sw, tiles, levels, st);
 }
 }  // namespace KVARIANT
 }  // namespace mgpu
@@ -1848,20 +1832,11 @@ int launch_fused_subgrid(const Scalars& s, DevState<T>& d, cudaStream_t st) {
     return 1;
   }
   const size_t smem = tiled::smag_smem<T>();
-  static int occ = 0, nsm = 0;
-  if (!nsm) {
-    cudaFuncSetAttribute(k_f_smag_tiled<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    cudaFuncSetAttribute(k_f_smag_tiled<T>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_f_smag_tiled<T>, tiled::NT, smem);
-    int dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-    if (occ < 1) occ = 1;
-    if (nsm < 1) nsm = 1;
-  }
+  static LaunchTable table;
+  const LaunchLimits lim = launch_limits(table, {(const void*)k_f_smag_tiled<T>}, tiled::NT, smem);
   k_c_lower_bc<T><<<dim3((s.nx + 31) / 32, (s.ny + 7) / 8, 1), pt_block(), 0, st>>>(s, d);
   const int tiles = (s.nx / tiled::TX) * (s.ny / tiled::TY), levels = s.nz - 2;
-  const int nc = s.level_chunks > 0 ? s.level_chunks : choose_level_chunks(tiles, occ * nsm, levels);
+  const int nc = s.level_chunks > 0 ? s.level_chunks : choose_level_chunks(tiles, lim.occ * lim.nsm, levels);
   const int kc = (levels + nc - 1) / nc;
   dim3 grid(s.nx / tiled::TX, s.ny / tiled::TY, (levels + kc - 1) / kc);
   k_f_smag_tiled<T><<<grid, dim3(tiled::TX, tiled::TY, 1), smem, st>>>(s, d, kc);
@@ -1889,24 +1864,14 @@ int launch_fused_dynamics(const Scalars& s, DevState<T>& d, cudaStream_t st, cud
     return 1;
   }
   const size_t sm_m = tiled::momentum_smem<T>();
-  static int occ_m = 0, nsm = 0;
-  if (!nsm) {
-    cudaFuncSetAttribute(k_f_momentum_tiled<T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_m);
-    cudaFuncSetAttribute(k_f_momentum_tiled<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_m);
-    cudaFuncSetAttribute(k_f_momentum_tiled<T, false>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
-    cudaFuncSetAttribute(k_f_momentum_tiled<T, true>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_m, k_f_momentum_tiled<T, false>, tiled::NT, sm_m);
-    int dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-    if (occ_m < 1) occ_m = 1;
-    if (nsm < 1) nsm = 1;
-  }
+  static LaunchTable table;
+  const LaunchLimits lim = launch_limits(
+      table, {(const void*)k_f_momentum_tiled<T, false>, (const void*)k_f_momentum_tiled<T, true>}, tiled::NT, sm_m);
   const int tiles = (s.nx / tiled::TX) * (s.ny / tiled::TY), levels = s.nz - 1;
-  int nl = launch_scalar_part<T>(s, d, tiles, nsm, levels, st);
+  int nl = launch_scalar_part<T>(s, d, tiles, levels, st);
   if (mid) cudaEventRecord(mid, st);
-  if (s.tvd_flow) nl += launch_flow_part<T>(s, d, tiles, nsm, levels, st);
-  const int nc_m = s.level_chunks > 0 ? s.level_chunks : choose_level_chunks(tiles, occ_m * nsm, levels);
+  if (s.tvd_flow) nl += launch_flow_part<T>(s, d, tiles, levels, st);
+  const int nc_m = s.level_chunks > 0 ? s.level_chunks : choose_level_chunks(tiles, lim.occ * lim.nsm, levels);
   const int kc_m = (levels + nc_m - 1) / nc_m;
   dim3 block(tiled::TX, tiled::TY, 1);
   dim3 grid_m(s.nx / tiled::TX, s.ny / tiled::TY, (levels + kc_m - 1) / kc_m);

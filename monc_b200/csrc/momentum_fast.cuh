@@ -334,21 +334,11 @@ __global__ void __launch_bounds__(NT, ctas<T>()) k_f_momentum(const __grid_const
 template <typename T>
 static int launch(const Scalars& s, DevState<T>& d, cudaStream_t st) {
   const size_t smem = smem_bytes<T, false>();
-  static int occ = 0, nsm = 0;
-  if (!nsm) {
-    cudaFuncSetAttribute(k_f_momentum<T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    cudaFuncSetAttribute(k_f_momentum<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    cudaFuncSetAttribute(k_f_momentum<T, false>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
-    cudaFuncSetAttribute(k_f_momentum<T, true>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_f_momentum<T, false>, NT, smem);
-    if (occ < 1) occ = 1;
-    int dev = 0, n = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-    nsm = n < 1 ? 1 : n;
-  }
+  static LaunchTable table;
+  const LaunchLimits lim =
+      launch_limits(table, {(const void*)k_f_momentum<T, false>, (const void*)k_f_momentum<T, true>}, NT, smem);
   const int gx = (s.nx + TX - 1) / TX, gy = (s.ny + TY - 1) / TY, levels = s.nz - 1;
-  const int nc = s.level_chunks > 0 ? s.level_chunks : tvdf::choose_chunks(gx * gy, occ, nsm, levels);
+  const int nc = s.level_chunks > 0 ? s.level_chunks : tvdf::choose_chunks(gx * gy, lim.occ, lim.nsm, levels);
   const int kc = (levels + nc - 1) / nc;
   const dim3 grid(gx, gy, (levels + kc - 1) / kc);
   if (s.tvd_flow) k_f_momentum<T, true><<<grid, NT, smem, st>>>(s, d, kc);

@@ -280,19 +280,10 @@ __global__ void __launch_bounds__(NT, ctas<T>()) k_f_smag(const __grid_constant_
 template <typename T, bool MOIST>
 static int launch_as(const Scalars& s, DevState<T>& d, cudaStream_t st) {
   const size_t smem = smem_bytes<T>();
-  static int occ = 0, nsm = 0;
-  if (!nsm) {
-    cudaFuncSetAttribute(k_f_smag<T, MOIST>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    cudaFuncSetAttribute(k_f_smag<T, MOIST>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_f_smag<T, MOIST>, NT, smem);
-    if (occ < 1) occ = 1;
-    int dev = 0, n = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-    nsm = n < 1 ? 1 : n;
-  }
+  static LaunchTable table;
+  const LaunchLimits lim = launch_limits(table, {(const void*)k_f_smag<T, MOIST>}, NT, smem);
   const int gx = (s.nx + TX - 1) / TX, gy = (s.ny + TY - 1) / TY, levels = s.nz - 2;
-  const int nc = s.level_chunks > 0 ? s.level_chunks : tvdf::choose_chunks(gx * gy, occ, nsm, levels);
+  const int nc = s.level_chunks > 0 ? s.level_chunks : tvdf::choose_chunks(gx * gy, lim.occ, lim.nsm, levels);
   const int kc = (levels + nc - 1) / nc;
   k_f_smag<T, MOIST><<<dim3(gx, gy, 1 + (levels + kc - 1) / kc), NT, smem, st>>>(s, d, kc);
   return 1;

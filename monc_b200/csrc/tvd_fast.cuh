@@ -703,19 +703,10 @@ static inline int choose_chunks(int tiles, int occ, int nsm, int levels) {
 template <typename T, int NS, bool CLOUD, int DIM>
 static int launch(const Scalars& s, const Job<T, NS>& job, cudaStream_t st) {
   const size_t smem = smem_bytes<T, NS, DIM>();
-  static int occ = 0, nsm = 0;
-  if (!nsm) {
-    cudaFuncSetAttribute(k_f_tvd<T, NS, CLOUD, DIM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    cudaFuncSetAttribute(k_f_tvd<T, NS, CLOUD, DIM>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_f_tvd<T, NS, CLOUD, DIM>, NT, smem);
-    if (occ < 1) occ = 1;
-    int dev = 0, n = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-    nsm = n < 1 ? 1 : n;
-  }
+  static LaunchTable table;
+  const LaunchLimits lim = launch_limits(table, {(const void*)k_f_tvd<T, NS, CLOUD, DIM>}, NT, smem);
   const int gx = (s.nx + TX - 1) / TX, gy = (s.ny + TY - 1) / TY, levels = s.nz - 1;
-  const int nc = s.level_chunks > 0 ? s.level_chunks : choose_chunks(gx * gy, occ, nsm, levels);
+  const int nc = s.level_chunks > 0 ? s.level_chunks : choose_chunks(gx * gy, lim.occ, lim.nsm, levels);
   const int kc = (levels + nc - 1) / nc;
   k_f_tvd<T, NS, CLOUD, DIM><<<dim3(gx, gy, (levels + kc - 1) / kc), NT, smem, st>>>(s, job, kc);
   return 1;
