@@ -13,7 +13,6 @@
 // pencilfft.F90:276-332); the solve is linear with real coefficients that depend only on
 // |kx|, |ky|, so this complex half-spectrum form gives the same field up to rounding.
 // Level 1 is transformed too: its non-mean modes pass through unchanged, its mean is zeroed.
-#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -25,6 +24,7 @@
 #include <mutex>
 
 #include "dycore.h"
+#include "level_sums.cuh"
 
 namespace mgpu {
 
@@ -1581,12 +1581,8 @@ template void slab_solve_columns<float>(const FftPlanDev&, const Scalars&, void*
                                         int64_t*);
 
 // ---- horizontal-mean diagnostics: one cluster of blocks per level, FP64 accumulation in a fixed order ----
-// Level sums split over a cluster of PSPLIT blocks (one cluster per level): block r sums its
-// contiguous share of the level's points, each thread in a fixed stride order and the block by a
-// tree; block 0 then adds the PSPLIT partial sums in rank order through distributed shared memory.
-// Deterministic, and a level keeps PSPLIT blocks busy where one block per level left most of the
-// GPU idle.
-constexpr int PSPLIT = 8, PRED_T = 256;
+// (level_sums.cuh; each thread sums in a fixed stride order and the block by a tree)
+constexpr int PRED_T = 256;
 
 template <int NV>
 __device__ __forceinline__ void block_tree(double (*sh)[PRED_T]) {
@@ -1597,24 +1593,6 @@ __device__ __forceinline__ void block_tree(double (*sh)[PRED_T]) {
       for (int q = 0; q < NV; ++q) sh[q][threadIdx.x] += sh[q][threadIdx.x + h];
     __syncthreads();
   }
-}
-
-// the cluster's total of sh[q][0] over its blocks, valid in block 0 (thread 0)
-template <int NV>
-__device__ __forceinline__ void cluster_total(double (*sh)[PRED_T], double* tot) {
-  namespace cg = cooperative_groups;
-  cg::cluster_group cluster = cg::this_cluster();
-  cluster.sync();
-  if (cluster.block_rank() == 0 && threadIdx.x == 0) {
-#pragma unroll
-    for (int q = 0; q < NV; ++q) tot[q] = 0.0;
-    for (int r = 0; r < PSPLIT; ++r) {
-      double(*rs)[PRED_T] = cluster.map_shared_rank(sh, r);
-#pragma unroll
-      for (int q = 0; q < NV; ++q) tot[q] += rs[q][0];
-    }
-  }
-  cluster.sync();  // no block leaves while block 0 reads its partial sums
 }
 
 template <typename T>

@@ -7,18 +7,15 @@
 // fused step those are zu_n, zv_n and the new theta and q; the next step's damping and forcing
 // read them.  Each level of each field is summed in a fixed order (deterministic), in FP64 whatever
 // the field precision, and multiplied by rnhpts = 1 / real(nx ny) as MONC does.
-#include <cooperative_groups.h>
-
 #include "dycore.h"
 #include "dycore_device.cuh"
+#include "level_sums.cuh"
 
 namespace mgpu {
 
-// Level sums are split over a cluster of PSPLIT blocks, each a contiguous share of the level's points
-// in a fixed order; block 0 adds the shares in rank order through distributed shared memory.  (One block
-// per level left most of the chip idle and waited for one load per trip: the six profiles of
-// 128 x 128 x 96 in FP64 took 2 x 17.2 us, now 20.7 us in one launch: 88 MB, 4.3 TB/s.)
-constexpr int PSPLIT = 8, PT = 256;
+// Level sums over a cluster of blocks (level_sums.cuh).  One block per level waited for one load per trip:
+// the six profiles of 128 x 128 x 96 in FP64 took 2 x 17.2 us, now 20.7 us in one launch: 88 MB, 4.3 TB/s.
+constexpr int PT = 256;
 
 // sums v[q] of the block's threads (in place in thread 0): warp shuffles, then the warps in order
 template <int NV>
@@ -39,29 +36,12 @@ __device__ __forceinline__ void block_sums(double (&v)[NV], double (*sh)[PT / 32
       sh[q][0] = a;
     }
 }
-// the cluster's totals of sh[q][0], in thread 0 of block 0
-template <int NV>
-__device__ __forceinline__ void cluster_sums(double (*sh)[PT / 32], double (&tot)[NV]) {
-  namespace cg = cooperative_groups;
-  cg::cluster_group cluster = cg::this_cluster();
-  cluster.sync();
-  if (cluster.block_rank() == 0 && threadIdx.x == 0) {
-#pragma unroll
-    for (int q = 0; q < NV; ++q) tot[q] = 0.0;
-    for (int r = 0; r < PSPLIT; ++r) {
-      double(*rs)[PT / 32] = cluster.map_shared_rank(sh, r);
-#pragma unroll
-      for (int q = 0; q < NV; ++q) tot[q] += rs[q][0];
-    }
-  }
-  cluster.sync();  // no block leaves while block 0 reads its sums
-}
 
 // field q of a mean: c[q] + p[q], or a[q] p[q] + b[q] p2[q] when p2[q] is set (theta after
 // stepfields' time smoothing); row q of the result starts at out[q]
 constexpr int MAX_MEANS = 2 * (3 + MGPU_MAX_Q);
 template <typename T>
-struct MeanFields {
+struct MeanRows {
   const T* p[MAX_MEANS];
   const T* p2[MAX_MEANS];
   double a[MAX_MEANS], b[MAX_MEANS], c[MAX_MEANS];
@@ -72,7 +52,7 @@ struct MeanFields {
 // the level sums run over count points from row offset off of each plane (a slab's interior rows)
 template <typename T>
 __global__ void __cluster_dims__(PSPLIT, 1, 1) __launch_bounds__(PT)
-    k_plane_means(const __grid_constant__ MeanFields<T> f, long long plane, long long off, long long count, double rnhpts) {
+    k_plane_means(const __grid_constant__ MeanRows<T> f, long long plane, long long off, long long count, double rnhpts) {
   const int k = blockIdx.y + 1, q = blockIdx.z, r = blockIdx.x;
   const long long chunk = (count + PSPLIT - 1) / PSPLIT, t0 = r * chunk, t1 = min(count, t0 + chunk);
   const long long base = (long long)(k - 1) * plane + off;
@@ -90,7 +70,7 @@ __global__ void __cluster_dims__(PSPLIT, 1, 1) __launch_bounds__(PT)
   __shared__ double sh[1][PT / 32];
   block_sums<1>(acc, sh);
   double tot[1];
-  cluster_sums<1>(sh, tot);
+  cluster_total<1>(sh, tot);
   if (r == 0 && threadIdx.x == 0) f.out[q][k] = tot[0] * rnhpts;
 }
 
@@ -102,7 +82,7 @@ static double rnhpts(const Scalars& s, int halo) { return 1.0 / (double)(float)i
 
 // olzubar, olzvbar, olzthbar and olzqbar(n): the means of zu, zv, theta and the q fields
 template <typename T>
-static void add_olz(MeanFields<T>& f, const Scalars& s, const T* zu, const T* zv, const T* th, const T* const* q, double* olz) {
+static void add_olz(MeanRows<T>& f, const Scalars& s, const T* zu, const T* zv, const T* th, const T* const* q, double* olz) {
   const T* p[3] = {zu, zv, th};
   for (int n = 0; n < 3 + s.nq; ++n, ++f.n) {
     f.p[f.n] = n < 3 ? p[n] : q[n - 3];
@@ -112,7 +92,7 @@ static void add_olz(MeanFields<T>& f, const Scalars& s, const T* zu, const T* zv
 // olubar, olvbar, olthbar and olqbar(n): the means of ugal + u, vgal + v, theta and each q field,
 // the scalars time-smoothed (c1 f + c2 zf) where their z-fields are given
 template <typename T>
-static void add_olbar(MeanFields<T>& f, const Scalars& s, const T* u, const T* v, const T* th, const T* zth,
+static void add_olbar(MeanRows<T>& f, const Scalars& s, const T* u, const T* v, const T* th, const T* zth,
                       const T* const* q, const T* const* zq, double ugal, double vgal, double c1, double c2, double* olbar) {
   const int nq = q ? s.nq : 0;
   for (int n = 0; n < 3 + nq; ++n, ++f.n) {
@@ -130,7 +110,7 @@ static void add_olbar(MeanFields<T>& f, const Scalars& s, const T* u, const T* v
   }
 }
 template <typename T>
-static int launch_means(const MeanFields<T>& f, const Scalars& s, cudaStream_t st, int halo) {
+static int launch_means(const MeanRows<T>& f, const Scalars& s, cudaStream_t st, int halo) {
   k_plane_means<T><<<dim3(PSPLIT, s.nz, f.n), PT, 0, st>>>(f, s.plane, (long long)halo * s.nx, interior(s, halo),
                                                            rnhpts(s, halo));
   return 1;
@@ -139,7 +119,7 @@ static int launch_means(const MeanFields<T>& f, const Scalars& s, cudaStream_t s
 template <typename T>
 int launch_mean_profiles(const Scalars& s, const MeanProfileFields<T>& m, double* olz, double* olbar, cudaStream_t st,
                          int halo) {
-  MeanFields<T> f{};
+  MeanRows<T> f{};
   add_olz(f, s, m.zu, m.zv, m.zs, m.zqs, olz);
   add_olbar(f, s, m.u, m.v, m.th, m.zth, m.q, m.zq, m.ugal, m.vgal, m.c1, m.c2, olbar);
   return launch_means(f, s, st, halo);
@@ -209,7 +189,7 @@ __global__ void __cluster_dims__(PSPLIT, 1, 1) __launch_bounds__(PT) k_profile_d
   __shared__ double sh[NR][PT / 32];
   block_sums<NR>(acc, sh);
   double tot[NR];
-  cluster_sums<NR>(sh, tot);
+  cluster_total<NR>(sh, tot);
   const int nrows = moist ? NR : MGPU_PD_VAPOUR;
   if (r0 == 0 && threadIdx.x == 0)
     for (int r = 0; r < nrows; ++r) out[(size_t)r * nz + k - 1] = tot[r];
