@@ -548,6 +548,11 @@ int mgpu_slab_cfl_extrema(mgpu_handle* h, double* d_buf, int32_t put, int32_t* g
 #define MGPU_SLAB_ITER_INNER     13
 #define MGPU_SLAB_ITER_CORRECT   14
 #define MGPU_SLAB_ITER_UNCORRECT 15
+/* PREPARE, once after mgpu_slab_init and before the first phase: says that this slab's pressure is
+ * solved by these steps and sets the solver up (BEGIN does both where it was not called, after
+ * the first dynamics).  The fast build's phases then run the kernels that mgpu_step runs for
+ * solver MGPU_SOLVER_ITERATIVE, and a decomposed run takes the single domain's values. */
+#define MGPU_SLAB_ITER_PREPARE   16
 /* solver_type MGPU_ITER_CG (MONC's default; the symmetric form of the operator):
  *
  *   BEGIN; halo exchange of MGPU_HALO_ITER_X; INIT, sum, FINISH     r = b A_vol - A x

@@ -1574,13 +1574,15 @@ int mgpu_slab_iter(mgpu_handle* h, int32_t step, double* d_sums, int32_t* done) 
   if (!h->slab_halo) return fail(h, MGPU_ERR_ARGUMENT, "mgpu_slab_init first");
   const size_t n = field_elems(h);
   void* p = h->fp32 ? static_cast<void*>(h->d32.p) : static_cast<void*>(h->d64.p);
-  if (step == MGPU_SLAB_ITER_BEGIN) {
+  if (step == MGPU_SLAB_ITER_BEGIN || step == MGPU_SLAB_ITER_PREPARE) {
     if (!h->iter) {
       int st = MGPU_OK;
       h->iter = iter_create(h->sc, h->rs, h->cfg, h->fp32, &st, h->slab_halo, h->cfg.ny - h->slab_halo,
                             h->slab_ny_global);
       if (st) return fail(h, st, "iterative solver setup");
+      h->sc.krylov = 1;  // the slab's phases run the kernels that the single domain's steps run
     }
+    if (step == MGPU_SLAB_ITER_PREPARE) return MGPU_OK;
     if (int rc = iter_slab_begin(h->iter, p, n, h->stream)) return fail(h, rc, "slab iterative begin");
     return MGPU_OK;
   }

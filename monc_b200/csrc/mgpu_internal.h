@@ -77,7 +77,8 @@ struct Scalars {
   int point_dynamics;  // 1: always use the untiled dynamics kernel (MGPU_POINT_DYNAMICS=1)
   int level_chunks;    // level chunks of the tiled dynamics kernels; 0 = chosen from the occupancy
                        // (MGPU_LEVEL_CHUNKS=n fixes it)
-  int krylov;          // 1: the pressure solver is iterative.  Its iterates amplify rounding (a cold solve of
+  int krylov;          // 1: the pressure solver is iterative (solver MGPU_SOLVER_ITERATIVE, or a slab's
+                       // MGPU_SLAB_ITER_PREPARE).  Its iterates amplify rounding (a cold solve of
                        // some hundred iterations turns 1e-14 in the source into 3e-3 in the pressure it
                        // stops at), so the contracted build keeps to one set of kernels, the ones it
                        // shares with the separately rounded build, for these models

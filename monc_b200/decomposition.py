@@ -315,6 +315,8 @@ class SlabDomain:
             c.solver = cf.SOLVER_EXTERNAL
             m = api.Model(c)
             m.slab_init(g.ny, halo, max(w for _, w in g.blocks))
+            if self.iterative:
+                m.slab_iter(cf.SLAB_ITER_PREPARE)
             self.slabs.append(_Slab(r, m, g, dtype, self.device))
         if isinstance(comm, TorchComm) and self.device.type == "cuda":
             comm.stream = torch.cuda.ExternalStream(self.slabs[0].m.stream, device=self.device)

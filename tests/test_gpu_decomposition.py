@@ -593,3 +593,28 @@ def test_torch_comm_over_nccl_single_rank(gpu_lib, precision, mode):
     r = subprocess.run([sys.executable, "-c", NCCL_ONE_RANK, str(precision), mode], cwd=root, env=env,
                        capture_output=True, text=True, timeout=300)
     assert r.returncode == 0 and "SLAB-NCCL-OK" in r.stdout, r.stdout[-2000:] + r.stderr[-2000:]
+
+
+@ITER_TYPES
+@pytest.mark.parametrize("timestep", [1, 2], ids=["forward", "centred"])
+def test_contracted_iterative_slabs_run_the_single_domain_kernels(gpu_lib, monkeypatch, timestep, stype):
+    """What a step computes before its pressure solve -- viscosity, diffusivity, theta -- is the single
+    domain's bit for bit in the contracted build too: the slabs of an iterative model run the same kernels."""
+    monkeypatch.setenv("MGPU_LEVEL_CHUNKS", "2")  # the same split of the levels on both sides
+    c = iterative_config(1e-30, 2, stype)
+    c.reproducible = 0
+    st = dry_state()
+    fields = ["vis", "diff", "th", "zth"]
+    m = api.Model(c)
+    m.set_state(st)
+    m.set_timestep(timestep)
+    m.step(1)
+    ref = {f: m.download(f) for f in fields}
+    m.close()
+    d = dc.SlabDomain(c, dc.LoopbackComm(2))
+    d.set_state(st)
+    d.set_timestep(timestep)
+    d.step(1)
+    for f in fields:
+        np.testing.assert_array_equal(d.download(f), ref[f], err_msg=f)
+    d.close()
