@@ -13,8 +13,7 @@
 
 namespace mgpu {
 
-// Level sums over a cluster of blocks (level_sums.cuh).  One block per level waited for one load per trip:
-// the six profiles of 128 x 128 x 96 in FP64 took 2 x 17.2 us, now 20.7 us in one launch: 88 MB, 4.3 TB/s.
+// Level sums over a cluster of blocks (level_sums.cuh); all profiles of a step in one launch.
 constexpr int PT = 256;
 
 // sums v[q] of the block's threads (in place in thread 0): warp shuffles, then the warps in order
@@ -37,6 +36,40 @@ __device__ __forceinline__ void block_sums(double (&v)[NV], double (*sh)[PT / 32
     }
 }
 
+// How many blocks (1, 2, 4 or 8) share a level of `points` points, for `sums` level sums in all: the number
+// with the least waves x (a block's points + `fixed`), fixed standing for what a block costs besides its
+// points and 5% a doubling for the cluster.  FP64, a call with its wait, for 1, 2, 4, 8 blocks, [chosen]:
+//   six means    64 x 64 x 1000 [47] 53 74 155, 256 x 128 x 60 32 [23] 25 26, 1024 x 1024 x 20 603 322 192 [156] us
+//   diagnostics  64 x 64 x 1000 [93] 101 120 181, 256 x 128 x 60 95 70 [46] 58, 1024 x 1024 x 20 4663 2368 1173 [619]
+// (always eight blocks lost on deep grids of small levels, one block on few or large levels).  `slots` are the
+// blocks resident on the 148 SMs of a B200, a constant so that the order of the sums does not depend on the device.
+constexpr int SPLIT_SMS = 148;
+static int level_split(long long points, long long sums, int slots, double fixed) {
+  int best = 1;
+  double best_cost = 0.0, penalty = 1.0;
+  for (int n = 1; n <= PSPLIT; n *= 2, penalty += 0.05) {
+    const long long waves = (sums * n + slots - 1) / slots;
+    const double cost = (double)waves * ((double)points / n + fixed) * penalty;
+    if (n == 1 || cost < best_cost) { best = n; best_cost = cost; }
+  }
+  return best;
+}
+// kernel on `split` blocks a cluster for each of levels x rows sums
+template <typename... P, typename... A>
+static void launch_split(void (*kernel)(P...), int split, int levels, int rows, cudaStream_t st, A... args) {
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = split;
+  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(split, levels, rows);
+  cfg.blockDim = dim3(PT, 1, 1);
+  cfg.stream = st;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
 // field q of a mean: c[q] + p[q], or a[q] p[q] + b[q] p2[q] when p2[q] is set (theta after
 // stepfields' time smoothing); row q of the result starts at out[q]
 constexpr int MAX_MEANS = 2 * (3 + MGPU_MAX_Q);
@@ -51,10 +84,10 @@ struct MeanRows {
 
 // the level sums run over count points from row offset off of each plane (a slab's interior rows)
 template <typename T>
-__global__ void __cluster_dims__(PSPLIT, 1, 1) __launch_bounds__(PT)
+__global__ void __launch_bounds__(PT)
     k_plane_means(const __grid_constant__ MeanRows<T> f, long long plane, long long off, long long count, double rnhpts) {
-  const int k = blockIdx.y + 1, q = blockIdx.z, r = blockIdx.x;
-  const long long chunk = (count + PSPLIT - 1) / PSPLIT, t0 = r * chunk, t1 = min(count, t0 + chunk);
+  const int k = blockIdx.y + 1, q = blockIdx.z, r = blockIdx.x, split = gridDim.x;
+  const long long chunk = (count + split - 1) / split, t0 = r * chunk, t1 = min(count, t0 + chunk);
   const long long base = (long long)(k - 1) * plane + off;
   const T* __restrict__ p = f.p[q] + base;
   const T* __restrict__ p2 = f.p2[q] ? f.p2[q] + base : nullptr;
@@ -69,8 +102,8 @@ __global__ void __cluster_dims__(PSPLIT, 1, 1) __launch_bounds__(PT)
   }
   __shared__ double sh[1][PT / 32];
   block_sums<1>(acc, sh);
-  double tot[1];
-  cluster_total<1>(sh, tot);
+  double tot[1] = {sh[0][0]};
+  if (split > 1) cluster_total<1>(sh, tot);
   if (r == 0 && threadIdx.x == 0) f.out[q][k] = tot[0] * rnhpts;
 }
 
@@ -111,8 +144,8 @@ static void add_olbar(MeanRows<T>& f, const Scalars& s, const T* u, const T* v, 
 }
 template <typename T>
 static int launch_means(const MeanRows<T>& f, const Scalars& s, cudaStream_t st, int halo) {
-  k_plane_means<T><<<dim3(PSPLIT, s.nz, f.n), PT, 0, st>>>(f, s.plane, (long long)halo * s.nx, interior(s, halo),
-                                                           rnhpts(s, halo));
+  launch_split(k_plane_means<T>, level_split(interior(s, halo), (long long)s.nz * f.n, 8 * SPLIT_SMS, 16000.0), s.nz, f.n, st, f, s.plane,
+               (long long)halo * s.nx, interior(s, halo), rnhpts(s, halo));
   return 1;
 }
 
@@ -127,11 +160,12 @@ int launch_mean_profiles(const Scalars& s, const MeanProfileFields<T>& m, double
 template int launch_mean_profiles<float>(const Scalars&, const MeanProfileFields<float>&, double*, double*, cudaStream_t, int);
 template int launch_mean_profiles<double>(const Scalars&, const MeanProfileFields<double>&, double*, double*, cudaStream_t, int);
 
-// profile_diagnostics (profile_diagnostics.F90:311-636, PW flow and TVD scalars): one cluster
-// per level sums the MGPU_PD_* quantities over the plane in FP64, in a fixed order (one block per level:
-// 79 us at 128 x 128 x 96 in FP64, now 34 us)
+// profile_diagnostics (profile_diagnostics.F90:311-636, PW flow and TVD scalars): a level's blocks sum
+// the MGPU_PD_* quantities over the plane in FP64, in a fixed order.  Bound by its loads' latency: two points
+// a thread are in flight at three blocks an SM (80 registers; one point 5% slower, four blocks with one point
+// 20% faster where the levels alone fill the chip and 5% slower on large levels).
 template <typename T>
-__global__ void __cluster_dims__(PSPLIT, 1, 1) __launch_bounds__(PT) k_profile_diagnostics(Scalars s, const T* __restrict__ u,
+__global__ void __launch_bounds__(PT, 3) k_profile_diagnostics(Scalars s, const T* __restrict__ u,
                                                              const T* __restrict__ v, const T* __restrict__ w,
                                                              const T* __restrict__ th, const T* __restrict__ qv,
                                                              const T* __restrict__ ql, const double* __restrict__ olbar,
@@ -147,10 +181,17 @@ __global__ void __cluster_dims__(PSPLIT, 1, 1) __launch_bounds__(PT) k_profile_d
   const double thbar = olbar[2 * st + k];
   const double umean = (k < nz && has_mean) ? 0.5 * (olbar[k] + olbar[k + 1]) : 0.0;
   const double vmean = (k < nz && has_mean) ? 0.5 * (olbar[st + k] + olbar[st + k + 1]) : 0.0;
-  const long long count = (long long)s.nx * (s.ny - 2 * halo);
-  const long long chunk = (count + PSPLIT - 1) / PSPLIT, t1 = min(count, (r0 + 1) * chunk);
-  for (long long t = r0 * chunk + threadIdx.x; t < t1; t += PT) {
-    const int j = halo + (int)(t / s.nx), i = (int)(t % s.nx);
+  // (a level has fewer than 2^31 points; a thread's next point is PT points on, without a division)
+  const unsigned nx = s.nx, count = nx * (unsigned)(s.ny - 2 * halo);
+  const unsigned chunk = (count + gridDim.x - 1) / gridDim.x, t1 = min(count, (r0 + 1) * chunk);
+  const unsigned t0 = r0 * chunk + threadIdx.x, dj = PT / nx, di = PT % nx;
+  unsigned row = t0 / nx, ix = t0 - row * nx;
+#pragma unroll 2
+  for (unsigned t = t0; t < t1; t += PT) {
+    const int j = halo + (int)row, i = (int)ix;
+    row += dj;
+    ix += di;
+    if (ix >= nx) { ix -= nx; ++row; }
     const long long o = g.at(k, j, i);
     const double w0 = (double)w[o], th0 = (double)th[o];
     acc[MGPU_PD_U_WIND] += (double)u[o] + ugal;
@@ -188,18 +229,24 @@ __global__ void __cluster_dims__(PSPLIT, 1, 1) __launch_bounds__(PT) k_profile_d
   }
   __shared__ double sh[NR][PT / 32];
   block_sums<NR>(acc, sh);
-  double tot[NR];
-  cluster_total<NR>(sh, tot);
+  if (gridDim.x > 1) {
+    double tot[NR];
+    cluster_total<NR>(sh, tot);
+    if (r0 == 0 && threadIdx.x == 0)
+#pragma unroll
+      for (int r = 0; r < NR; ++r) sh[r][0] = tot[r];
+  }
   const int nrows = moist ? NR : MGPU_PD_VAPOUR;
   if (r0 == 0 && threadIdx.x == 0)
-    for (int r = 0; r < nrows; ++r) out[(size_t)r * nz + k - 1] = tot[r];
+    for (int r = 0; r < nrows; ++r) out[(size_t)r * nz + k - 1] = sh[r][0];
 }
 
 template <typename T>
 int launch_profile_diagnostics(const Scalars& s, const T* u, const T* v, const T* w, const T* th, const T* qv,
                                const T* ql, const double* olbar, bool has_mean, double* out, cudaStream_t st,
                                int halo) {
-  k_profile_diagnostics<T><<<dim3(PSPLIT, s.nz), PT, 0, st>>>(s, u, v, w, th, qv, ql, olbar, has_mean ? 1 : 0, halo, out);
+  launch_split(k_profile_diagnostics<T>, level_split(interior(s, halo), s.nz, 3 * SPLIT_SMS, 1000.0), s.nz, 1, st, s, u, v, w, th, qv, ql,
+               olbar, has_mean ? 1 : 0, halo, out);
   return 1;
 }
 template int launch_profile_diagnostics<float>(const Scalars&, const float*, const float*, const float*, const float*,

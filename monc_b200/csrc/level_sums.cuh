@@ -7,7 +7,7 @@
 
 namespace mgpu {
 
-constexpr int PSPLIT = 8;  // blocks of a cluster
+constexpr int PSPLIT = 8;  // blocks of a cluster, at most
 
 // the cluster's total of sh[q][0] over its blocks, valid in block 0 (thread 0)
 template <int NV, int W>
@@ -18,7 +18,7 @@ __device__ __forceinline__ void cluster_total(double (*sh)[W], double* tot) {
   if (cluster.block_rank() == 0 && threadIdx.x == 0) {
 #pragma unroll
     for (int q = 0; q < NV; ++q) tot[q] = 0.0;
-    for (int r = 0; r < PSPLIT; ++r) {
+    for (int r = 0; r < (int)cluster.num_blocks(); ++r) {
       double(*rs)[W] = cluster.map_shared_rank(sh, r);
 #pragma unroll
       for (int q = 0; q < NV; ++q) tot[q] += rs[q][0];

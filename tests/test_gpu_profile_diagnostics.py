@@ -116,3 +116,52 @@ def test_field_value_retrieval_and_refusals(gpu_lib):
     with pytest.raises(api.MgpuError):
         m.profile_diagnostics()
     m.close()
+
+
+# grids whose levels are shared by 1, 2, 4 and 8 blocks, in the mean profiles and in the diagnostics;
+# shares that do not divide, and levels with fewer points than a block has threads
+SHARES = [(4, 4, 4), (6, 10, 300), (64, 64, 300), (32, 32, 128), (64, 36, 40), (128, 128, 8), (100, 100, 30),
+          (360, 300, 4), (250, 128, 60)]
+
+
+@pytest.mark.parametrize("grid", SHARES, ids=str)
+@pytest.mark.parametrize("precision", [cf.FP64, cf.FP32_MIXED], ids=["fp64", "fp32"])
+def test_level_sums_however_a_level_is_shared(gpu_lib, grid, precision):
+    """The mean profiles and the diagnostics against sums of the same fields in FP64: n terms summed in any
+    order are off by at most n 1.1e-16 of the sum of their magnitudes, which 1e-10 leaves room for
+    (n < 1.1e5)."""
+    nx, ny, nz = grid
+    c = cf.dry_cbl_config(nx, ny, nz, 50.0, 25.0, 0.5, ug=5.0, fcoriol=1e-4, precision=precision)
+    c.profile_diagnostics_enabled = 1
+    st = ini.random_flow_state(nx, ny, nz, seed=6, amp_uv=1.0, amp_w=0.3, amp_th=0.5, ug=5.0)
+    with api.Model(c) as m:
+        m.set_state(st)
+        m.component("mean_profiles")
+        f = {k: m.download(k) for k in api.STATE_FIELDS}
+        means, sums = m.mean_profiles(), m.profile_diagnostics()
+        thref = m.profile("thref")
+
+    def total(a):
+        return a.sum(axis=(1, 2)), np.abs(a).sum(axis=(1, 2))
+
+    def check(got, a, scale=1.0):
+        ref, mag = total(a)
+        assert np.all(np.abs(got - ref * scale) <= 1e-10 * mag * scale)
+
+    rn = 1.0 / float(np.float32(nx * ny))
+    for name, k in (("olzubar", "zu"), ("olzvbar", "zv"), ("olzthbar", "zth"), ("olubar", "u"), ("olvbar", "v"),
+                    ("olthbar", "th")):
+        check(means[name], f[k], rn)
+    u, v, w, th = (f[k] for k in ("u", "v", "w", "th"))
+    check(sums["u_wind_total_local"], u)
+    check(sums["v_wind_total_local"], v)
+    check(sums["ww_total_local"], w * w)
+    check(sums["theta_total_local"], th + thref[:, None, None])
+    check(sums["th2_total_local"], (th - means["olthbar"][:, None, None]) ** 2)
+    lo, hi = slice(1, nz - 1), slice(2, nz)
+    uw = 0.25 * (u[lo] + np.roll(u, 1, 2)[lo] + u[hi] + np.roll(u, 1, 2)[hi])
+    uw = (uw - 0.5 * (means["olubar"][lo] + means["olubar"][hi])[:, None, None]) * w[lo]
+    check(sums["uw_total_local"][lo], uw)
+    vw = 0.25 * (v[lo] + np.roll(v, 1, 1)[lo] + v[hi] + np.roll(v, 1, 1)[hi])
+    vw = (vw - 0.5 * (means["olvbar"][lo] + means["olvbar"][hi])[:, None, None]) * w[lo]
+    check(sums["vw_total_local"][lo], vw)
