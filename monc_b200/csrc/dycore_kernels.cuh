@@ -131,71 +131,84 @@ __global__ void k_c_pw(Scalars s, DevState<T> d) {
   if (k < s.nz) d.sw[o] = sw;
 }
 
-// tvd_advection of the flow fields (advect_flow_fields), which MONC does before theta's
-template <typename T>
-__global__ void k_c_tvd_flow(Scalars s, DevState<T> d) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  int j = blockIdx.y * blockDim.y + threadIdx.y;
-  int k = blockIdx.z + 2;
-  if (i >= s.nx || j >= s.ny || k > s.nz) return;
-  const Prof<T> P = prof<T>(s);
-  const long long o = lin(s, k, j, i);
-  const bool fwd = s.forward;
-  T su, sv, sw;
-  tvd_flow_point<T, View<T>>(s, P, view<T>(d.u, s), view<T>(d.v, s), view<T>(d.w, s), view<T>(fwd ? d.u : d.zu, s),
-                             view<T>(fwd ? d.v : d.zv, s), view<T>(fwd ? d.w : d.zw, s), k, j, i, d.su[o], d.sv[o],
-                             k < s.nz ? d.sw[o] : (T)0.0, su, sv, sw);
-  d.su[o] = su;
-  d.sv[o] = sv;
-  if (k < s.nz) d.sw[o] = sw;
-}
-
-// One tile of TVD_TX x TVD_TY columns marches up TVD_LEVELS levels of each scalar.  A face's flux is formed
+// tvd_advection: u, v, w where TVD carries the flow (advect_flow_fields), theta and each q field.
+//
+// One tile of TVD_TX x TVD_TY columns marches up L levels of a field.  A face's flux is formed
 // once, by the cell below or west of it: x and y faces pass through shared memory (two copies in turn, one
 // barrier a level), the z face is carried up, and only the tile's low sides and the chunk's lowest face are
-// formed twice.  Every face formed by both of its cells took 166 us for theta at 128 x 128 x 96 in FP64,
-// now 111 (128 with each warp forming its own low side; 113 at four blocks an SM, 117 with 16 levels); bound by
-// the faces' instructions.
-constexpr int TVD_TX = 32, TVD_TY = 8, TVD_LEVELS = 8;
+// formed twice.  Every face formed by both of its cells took 157 us for theta at 128 x 128 x 96 in FP64 (a call
+// with its wait), now 119 in eights; with TVD flow 776, or 1283 with u, v, w by points in a kernel of their own
+// (150 registers), now 569: three blocks an SM and 256 bytes of spills, 604 at two.  Bound by the faces' instructions.
+constexpr int TVD_TX = 32, TVD_TY = 8;
 template <typename T>
-__global__ void __launch_bounds__(TVD_TX * TVD_TY, 3) k_c_tvd(Scalars s, DevState<T> d) {
-  __shared__ T FX[2][TVD_TY][TVD_TX + 1], FY[2][TVD_TY + 1][TVD_TX];
+struct TvdFaces {
+  T x[2][TVD_TY][TVD_TX + 1], y[2][TVD_TY + 1][TVD_TX];
+};
+// the tile of one field: flow component DIM, advected on its dual grid, or with DIM = -1 a scalar;
+// levels kb .. ke
+template <typename T, int DIM>
+__device__ __forceinline__ void tvd_tile(const Scalars& s, const DevState<T>& d, const View<T>& ZF, T* src, int kb, int ke,
+                                         int& copy, TvdFaces<T>& sh) {
+  typedef typename std::conditional<DIM == 2, TvdMetricW, TvdMetricScalar>::type M;
+  typedef DualFlow<T, View<T>, DIM < 0 ? 0 : DIM> Dual;
+  typedef typename std::conditional<(DIM < 0), View<T>, Dual>::type A;
+  auto flow = [&](const T* p) -> A {
+    if constexpr (DIM < 0) return view<T>(p, s);
+    else return A{view<T>(p, s), s.nz};
+  };
+  const A U = flow(d.u), V = flow(d.v), W = flow(d.w);
   const int tx = threadIdx.x, ty = threadIdx.y;
   const int i0 = blockIdx.x * TVD_TX, j0 = blockIdx.y * TVD_TY, i = i0 + tx, j = j0 + ty;
-  const int kb = 2 + (int)blockIdx.z * TVD_LEVELS, ke = min(s.nz, kb + TVD_LEVELS - 1);
   const bool in = i < s.nx && j < s.ny;
   const Prof<T> P = prof<T>(s);
-  const View<T> U = view<T>(d.u, s), V = view<T>(d.v, s), W = view<T>(d.w, s);
-  const bool fwd = s.forward;
-  const T dt = (T)(s.dtm * 2.0);
-  int copy = 0;
-  // theta, then each q field (advect_theta, advect_q_fields)
-  for (int n = -1; n < s.nq; ++n) {
-    const View<T> ZF = view<T>(n < 0 ? (fwd ? d.th : d.zth) : (fwd ? d.q[n] : d.zq[n]), s);
-    T* const src = n < 0 ? d.sth : d.sq[n];
-    T fz_lo = in && kb > 2 ? tvd_face_z<T, View<T>>(s, P, U, V, W, ZF, dt, kb - 1, j, i) : (T)0.0;
-    for (int k = kb; k <= ke; ++k, copy ^= 1) {
-      const long long o = lin(s, k, j, i);
-      T acc = (T)0.0, fx = (T)0.0, fy = (T)0.0, fz_hi = (T)0.0;
-      if (in) {
-        acc = src[o];
-        fx = tvd_face_x<T, View<T>>(s, P, U, V, W, ZF, dt, k, j, i);
-        fy = tvd_face_y<T, View<T>>(s, P, U, V, W, ZF, dt, k, j, i);
-        if (k < s.nz) fz_hi = tvd_face_z<T, View<T>>(s, P, U, V, W, ZF, dt, k, j, i);
-        FX[copy][ty][tx + 1] = fx;
-        FY[copy][ty + 1][tx] = fy;
-      }
-      // the low sides: the first warp forms the row of y faces, the second the column of x faces
-      if (ty == 0 && i < s.nx) FY[copy][0][tx] = tvd_face_y<T, View<T>>(s, P, U, V, W, ZF, dt, k, j - 1, i);
-      if (ty == 1 && tx < TVD_TY && j0 + tx < s.ny)
-        FX[copy][tx][0] = tvd_face_x<T, View<T>>(s, P, U, V, W, ZF, dt, k, j0 + tx, i0 - 1);
-      __syncthreads();
-      if (in)
-        src[o] = tvd_source<T, View<T>>(s, P, U, V, W, FX[copy][ty][tx], fx, FY[copy][ty][tx], fy, fz_lo, fz_hi, k, j,
-                                        i, acc);
-      fz_lo = fz_hi;
-    }
+  const T dt = (T)(s.dtm * 2.0);  // (scalars and flow are always stepped centred, steppingdirection.F90:32)
+  T fz_lo = (T)0.0;
+  if (in) {
+    if (kb > 2) fz_lo = tvd_face_z<T, A, View<T>, Prof<T>, M>(s, P, U, V, W, ZF, dt, kb - 1, j, i);
+    else if constexpr (DIM == 2) fz_lo = tvd_face_z_bottom<T, A, View<T>, Prof<T>, M>(s, P, U, V, W, ZF, dt, j, i);
   }
+  for (int k = kb; k <= ke; ++k, copy ^= 1) {
+    const long long o = lin(s, k, j, i);
+    T acc = (T)0.0, fx = (T)0.0, fy = (T)0.0, fz_hi = (T)0.0;
+    if (in) {
+      acc = src[o];
+      fx = tvd_face_x<T, A, View<T>, Prof<T>, M>(s, P, U, V, W, ZF, dt, k, j, i);
+      fy = tvd_face_y<T, A, View<T>, Prof<T>, M>(s, P, U, V, W, ZF, dt, k, j, i);
+      if (k < s.nz) fz_hi = tvd_face_z<T, A, View<T>, Prof<T>, M>(s, P, U, V, W, ZF, dt, k, j, i);
+      sh.x[copy][ty][tx + 1] = fx;
+      sh.y[copy][ty + 1][tx] = fy;
+    }
+    // the low sides: the first warp forms the row of y faces, the second the column of x faces
+    if (ty == 0 && i < s.nx) sh.y[copy][0][tx] = tvd_face_y<T, A, View<T>, Prof<T>, M>(s, P, U, V, W, ZF, dt, k, j - 1, i);
+    if (ty == 1 && tx < TVD_TY && j0 + tx < s.ny)
+      sh.x[copy][tx][0] = tvd_face_x<T, A, View<T>, Prof<T>, M>(s, P, U, V, W, ZF, dt, k, j0 + tx, i0 - 1);
+    __syncthreads();
+    if (in)
+      src[o] = tvd_source<T, A, Prof<T>, M>(s, P, U, V, W, sh.x[copy][ty][tx], fx, sh.y[copy][ty][tx], fy, fz_lo, fz_hi, k, j,
+                                            i, acc);
+    fz_lo = fz_hi;
+  }
+}
+// blockIdx.z: with FLOW the chunks of u, v and w, then those of the scalars
+template <typename T, int L, bool FLOW, int CTAS>
+__global__ void __launch_bounds__(TVD_TX * TVD_TY, CTAS) k_c_tvd(Scalars s, DevState<T> d) {
+  __shared__ TvdFaces<T> sh;
+  const bool fwd = s.forward;
+  int chunk = blockIdx.z, copy = 0;
+  if constexpr (FLOW) {
+    const int n = (s.nz - 1 + L - 1) / L, dim = chunk / n;
+    const int kb = 2 + (chunk - dim * n) * L;
+    if (dim == 0) return tvd_tile<T, 0>(s, d, view<T>(fwd ? d.u : d.zu, s), d.su, kb, min(s.nz, kb + L - 1), copy, sh);
+    if (dim == 1) return tvd_tile<T, 1>(s, d, view<T>(fwd ? d.v : d.zv, s), d.sv, kb, min(s.nz, kb + L - 1), copy, sh);
+    // (w has no source at the top level)
+    if (dim == 2) return tvd_tile<T, 2>(s, d, view<T>(fwd ? d.w : d.zw, s), d.sw, kb, min(s.nz - 1, kb + L - 1), copy, sh);
+    chunk -= 3 * n;
+  }
+  const int kb = 2 + chunk * L, ke = min(s.nz, kb + L - 1);
+  // theta, then each q field (advect_theta, advect_q_fields)
+  for (int n = -1; n < s.nq; ++n)
+    tvd_tile<T, -1>(s, d, view<T>(n < 0 ? (fwd ? d.th : d.zth) : (fwd ? d.q[n] : d.zq[n]), s), n < 0 ? d.sth : d.sq[n], kb,
+                    ke, copy, sh);
 }
 
 // th_advection: the mean-baroclinicity term added to sth, levels 2..nz
@@ -1685,6 +1698,18 @@ __global__ void __launch_bounds__(256) k_f_pstep_swap(Scalars s, DevState<T> d) 
 // ==========================================================================================
 // host launchers
 // ==========================================================================================
+template <typename T, int L, int CTAS>
+static void launch_tvd_levels(const Scalars& s, const DevState<T>& d, int gx, int gy, cudaStream_t st) {
+  const int n = (s.nz - 1 + L - 1) / L;
+  const dim3 block(TVD_TX, TVD_TY, 1);
+  if (s.tvd_flow) k_c_tvd<T, L, true, CTAS><<<dim3(gx, gy, 4 * n), block, 0, st>>>(s, d);
+  else k_c_tvd<T, L, false, CTAS><<<dim3(gx, gy, n), block, 0, st>>>(s, d);
+}
+template <typename T>
+static void launch_tvd_component(const Scalars& s, const DevState<T>& d, cudaStream_t st) {
+  const int gx = (s.nx + TVD_TX - 1) / TVD_TX, gy = (s.ny + TVD_TY - 1) / TVD_TY;
+  launch_tvd_levels<T, 8, 3>(s, d, gx, gy, st);
+}
 template <typename T>
 int launch_component(int cid, const Scalars& s, DevState<T>& d, cudaStream_t st, unsigned long long* divmax,
                      int64_t* launches) {
@@ -1695,15 +1720,7 @@ int launch_component(int cid, const Scalars& s, DevState<T>& d, cudaStream_t st,
     case MGPU_C_LOWER_BC: k_c_lower_bc<T><<<gcol, b, 0, st>>>(s, d); break;
     case MGPU_C_SMAGORINSKY: k_c_smagorinsky<T><<<pt_grid(s, s.nz - 1), b, 0, st>>>(s, d); break;
     case MGPU_C_PW_ADVECTION: k_c_pw<T><<<pt_grid(s, s.nz - 1), b, 0, st>>>(s, d); break;
-    case MGPU_C_TVD_ADVECTION: 
-      if (s.tvd_flow) {
-        k_c_tvd_flow<T><<<pt_grid(s, s.nz - 1), b, 0, st>>>(s, d);
-        ++nl;
-      }
-      k_c_tvd<T><<<dim3((s.nx + TVD_TX - 1) / TVD_TX, (s.ny + TVD_TY - 1) / TVD_TY,
-                        (s.nz - 1 + TVD_LEVELS - 1) / TVD_LEVELS),
-                   dim3(TVD_TX, TVD_TY, 1), 0, st>>>(s, d);
-      break;
+    case MGPU_C_TVD_ADVECTION: launch_tvd_component<T>(s, d, st); break;
     case MGPU_C_DIFFUSION: k_c_diffusion<T><<<pt_grid(s, s.nz - 1), b, 0, st>>>(s, d); break;
     case MGPU_C_TH_ADVECTION:
       if (s.th_baroclinic) k_c_th_advection<T><<<pt_grid(s, s.nz - 1), b, 0, st>>>(s, d);
