@@ -137,8 +137,8 @@ __global__ void k_c_pw(Scalars s, DevState<T> d) {
 // once, by the cell below or west of it: x and y faces pass through shared memory (two copies in turn, one
 // barrier a level), the z face is carried up, and only the tile's low sides and the chunk's lowest face are
 // formed twice.  Every face formed by both of its cells took 157 us for theta at 128 x 128 x 96 in FP64 (a call
-// with its wait), now 119 in eights; with TVD flow 776, or 1283 with u, v, w by points in a kernel of their own
-// (150 registers), now 569: three blocks an SM and 256 bytes of spills, 604 at two.  Bound by the faces' instructions.
+// with its wait), now 108; with TVD flow 776, or 1283 with u, v, w by points in a kernel of their own
+// (150 registers), now 567: three blocks an SM and 256 bytes of spills, 604 at two.  Bound by the faces' instructions.
 constexpr int TVD_TX = 32, TVD_TY = 8;
 template <typename T>
 struct TvdFaces {
@@ -1705,10 +1705,20 @@ static void launch_tvd_levels(const Scalars& s, const DevState<T>& d, int gx, in
   if (s.tvd_flow) k_c_tvd<T, L, true, CTAS><<<dim3(gx, gy, 4 * n), block, 0, st>>>(s, d);
   else k_c_tvd<T, L, false, CTAS><<<dim3(gx, gy, n), block, 0, st>>>(s, d);
 }
+// The levels of a tile's march: 8 where that leaves enough blocks for 5 waves, so that the last one weighs
+// little (512 x 512 x 100 in FP64: 1705 us, 4 levels 1732), 4 or 2 from two waves on (64 x 64 x 300: 87 us in fours,
+// 94 in twos and 99 in eights; 32 x 32 x 600: 54 in twos, 60 in fours), and one level on smaller grids, where the
+// march is the time (32 x 32 x 32: 46 us in eights, 22 in twos, 17 in ones).  Grids of one wave also take
+// the registers of two blocks an SM (32 x 32 x 32: 16.5 us, three blocks 16.9; 64 x 64 x 65: 34 and 31).
 template <typename T>
 static void launch_tvd_component(const Scalars& s, const DevState<T>& d, cudaStream_t st) {
   const int gx = (s.nx + TVD_TX - 1) / TVD_TX, gy = (s.ny + TVD_TY - 1) / TVD_TY;
-  launch_tvd_levels<T, 8, 3>(s, d, gx, gy, st);
+  const long long tiles = (long long)gx * gy * (s.tvd_flow ? 4 : 1), levels = s.nz - 1;
+  if (tiles * ((levels + 7) / 8) >= 2500) launch_tvd_levels<T, 8, 3>(s, d, gx, gy, st);
+  else if (tiles * ((levels + 3) / 4) >= 900) launch_tvd_levels<T, 4, 3>(s, d, gx, gy, st);
+  else if (tiles * ((levels + 1) / 2) >= 900) launch_tvd_levels<T, 2, 3>(s, d, gx, gy, st);
+  else if (tiles * levels > 2 * 148) launch_tvd_levels<T, 1, 3>(s, d, gx, gy, st);
+  else launch_tvd_levels<T, 1, 2>(s, d, gx, gy, st);
 }
 template <typename T>
 int launch_component(int cid, const Scalars& s, DevState<T>& d, cudaStream_t st, unsigned long long* divmax,
