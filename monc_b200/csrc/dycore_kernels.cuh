@@ -1869,11 +1869,19 @@ int launch_fused_subgrid(const Scalars& s, DevState<T>& d, cudaStream_t st) {
   k_f_smag_tiled<T><<<grid, dim3(tiled::TX, tiled::TY, 1), smem, st>>>(s, d, kc);
   return 2;
 }
+// Grids of so few points that one launch with a thread a point beats the tiles' two to five launches: a step
+// of 4 x 4 x 8 in FP64 takes 39 us (tiles 46), with TVD flow 51 (74); TVD flow on 16 x 16 x 16 96 (103).  Above
+// 16 blocks of points, 64 with TVD flow, the tiles catch up (dry 8 x 8 x 32 55 and 58, moist 65 and 64).
+// Level chunks that are fixed by hand ask for the tiles.
+static inline bool few_points(const Scalars& s) {
+  const long long blocks = (long long)((s.nx + 31) / 32) * ((s.ny + 7) / 8) * s.nz;
+  return s.level_chunks == 0 && blocks <= (s.tvd_flow ? 64 : 16);
+}
 template <typename T>
 int launch_fused_dynamics(const Scalars& s, DevState<T>& d, cudaStream_t st, cudaEvent_t mid) {
 #ifdef MGPU_CONTRACTED
   // centred steps, any horizontal size
-  if (!s.forward && !s.point_dynamics && !s.krylov && (!s.tvd_flow || (d.su && d.sv && d.sw))) {
+  if (!s.forward && !s.point_dynamics && !s.krylov && !few_points(s) && (!s.tvd_flow || (d.su && d.sv && d.sw))) {
     int n = tvdf::launch_all_scalars<T>(s, d, st);
     if (mid) cudaEventRecord(mid, st);
     if (s.tvd_flow) n += tvdf::launch_all_flow<T>(s, d, st);
@@ -1883,8 +1891,12 @@ int launch_fused_dynamics(const Scalars& s, DevState<T>& d, cudaStream_t st, cud
   // the tiled kernels cover centred steps on sizes their tiles divide; the first (forward) step and
   // other sizes use the point kernel
   const bool moist = s.nq > 0;
-  const bool tiled_ok = !s.forward && !s.point_dynamics && (s.nx % tiled::TX) == 0 && (s.ny % tiled::TY) == 0 &&
-                        s.nz >= 4 && (!moist || (d.sth && d.sq[s.nq - 1])) && (!s.tvd_flow || (d.su && d.sv && d.sw));
+  bool point = s.forward || s.point_dynamics;
+#ifdef MGPU_CONTRACTED
+  point = point || (!s.krylov && few_points(s));
+#endif
+  const bool tiled_ok = !point && (s.nx % tiled::TX) == 0 && (s.ny % tiled::TY) == 0 && s.nz >= 4 &&
+                        (!moist || (d.sth && d.sq[s.nq - 1])) && (!s.tvd_flow || (d.su && d.sv && d.sw));
   if (!tiled_ok) {
     k_f_dynamics<T><<<pt_grid(s, s.nz), pt_block(), 0, st>>>(s, d);
     if (mid) cudaEventRecord(mid, st);

@@ -57,8 +57,8 @@ OPTIONS = {
 }
 
 
-def final_fields(options, nq, flow, precision, reproducible):
-    nx, ny, nz = GRID
+def final_fields(options, nq, flow, precision, reproducible, grid=GRID):
+    nx, ny, nz = grid
     c = cf.dry_cbl_config(nx, ny, nz, 50.0, 40.0, 0.5, ug=3.0, fcoriol=1e-4, precision=precision)
     c.advection_flow_fields = flow
     if nq:
@@ -82,9 +82,9 @@ def final_fields(options, nq, flow, precision, reproducible):
         return {f: m.download(f) for f in api.STATE_FIELDS + [p + str(n) for n in range(nq) for p in ("q", "zq")]}
 
 
-def compare(options, nq, flow, precision):
-    ref = final_fields(options, nq, flow, precision, 1)
-    got = final_fields(options, nq, flow, precision, 0)
+def compare(options, nq, flow, precision, grid=GRID):
+    ref = final_fields(options, nq, flow, precision, 1, grid)
+    got = final_fields(options, nq, flow, precision, 0, grid)
     tol = 1e-12 if precision == cf.FP64 else 2e-4
     for f in ref:
         assert np.abs(ref[f] - got[f]).max() <= tol * np.abs(ref[f]).max(), f
@@ -109,3 +109,20 @@ def test_options_in_level_chunks(gpu_lib, monkeypatch, options, chunks):
     """The whole column in one chunk, and chunks of one level."""
     monkeypatch.setenv("MGPU_LEVEL_CHUNKS", str(chunks))
     compare(options, 2, cf.ADVECT_TVD, cf.FP64)
+
+
+# on both sides of the line below which a thread takes a point: 16 blocks of 32 x 8 points, 64 with TVD flow
+@pytest.mark.parametrize("flow,grid", [(cf.ADVECT_PW, (32, 8, 16)), (cf.ADVECT_PW, (32, 8, 17)),
+                                       (cf.ADVECT_PW, (36, 10, 4)), (cf.ADVECT_PW, (36, 10, 5)),
+                                       (cf.ADVECT_TVD, (4, 4, 64)), (cf.ADVECT_TVD, (4, 4, 65)),
+                                       (cf.ADVECT_TVD, (36, 10, 16)), (cf.ADVECT_TVD, (36, 10, 17))], ids=str)
+@pytest.mark.parametrize("nq", [0, 2])
+def test_grids_of_few_points(gpu_lib, nq, flow, grid):
+    compare("inviscid", nq, flow, cf.FP64, grid)
+
+
+@pytest.mark.parametrize("nq,flow", [(0, cf.ADVECT_PW), (2, cf.ADVECT_TVD)], ids=["dry", "moist-tvd"])
+def test_shortest_columns_on_tiles(gpu_lib, monkeypatch, nq, flow):
+    """Four levels on the tiles, which a fixed number of level chunks asks for."""
+    monkeypatch.setenv("MGPU_LEVEL_CHUNKS", "1")
+    compare("at-rest", nq, flow, cf.FP64, (36, 10, 4))
