@@ -27,6 +27,8 @@
 // for theta, 0.082 ms; what is left above that is issue and latency with 16 warps per SM.
 #pragma once
 
+#include "reciprocal.cuh"
+
 namespace mgpu {
 namespace KVARIANT {
 namespace tvdf {
@@ -96,21 +98,6 @@ __device__ __forceinline__ double positive(double x) {
   return __hiloint2double(h & m, __double2loint(x) & m);
 }
 __device__ __forceinline__ float positive(float x) { return x > 0.0f ? x : 0.0f; }
-// 1/x for x >= 1e-30: the hardware's approximation, refined by Newton's iteration to the working
-// precision without the special cases of a correctly rounded reciprocal (whose branches would
-// keep the faces of a level from being interleaved)
-__device__ __forceinline__ double rcp_newton(double x) {
-  double r;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
-  r = fma(r, fma(-x, r, 1.0), r);
-  return fma(r, fma(-x, r, 1.0), r);
-}
-__device__ __forceinline__ float rcp_newton(float x) {
-  float r;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
-  return fmaf(r, fmaf(-x, r, 1.0f), r);
-}
-
 // The limited face value for fc - fu = a, fd - fc = e, the unlimited face b less fc, and r1 = 1 / S
 // - 1 of the upwind cell's outflow Courant sum S.  The limiter's max(a, min(b, a / S, fd - fu)) on
 // magnitudes, less a: max(0, min(b, a r1, e)) in the direction of a, added to fc.  Where a and e
