@@ -127,7 +127,8 @@ static int alloc_state(mgpu_handle* h, DevState<T>& d) {
       if (rc) return rc;
     }
   }
-  // the moist centred step passes the scalar sources through memory (tiled kernels, one per scalar)
+  // the sources of theta and the q fields (above): the component path's, and those the separately rounded
+  // build's and the iterative models' moist step passes through memory (one tiled kernel per scalar)
   if (h->cfg.number_q_fields > 0) {
     int rc = alloc_field<T>(h, &d.sth);
     if (rc) return rc;

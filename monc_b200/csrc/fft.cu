@@ -1056,20 +1056,17 @@ __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_gr
 // fit an SM, so the 33,024 columns of a 256 x 256 grid are one wave on 148 SMs.
 constexpr int TRI_TB = 112, TRI_KC = 8, TRI_NS = 4;
 constexpr size_t TRI_SMEM = (size_t)TRI_NS * TRI_KC * TRI_TB * (sizeof(double2) + sizeof(double));
+// what the mean mode's block keeps (mean_mode_block)
+__host__ __device__ constexpr size_t mean_smem(int nz) { return (size_t)(nz + 2) * (sizeof(double2) + 2 * sizeof(double)); }
+static_assert(mean_smem(MGPU_MAX_NZ) <= TRI_SMEM && TRI_SMEM % 16 == 0, "the mean mode works in the staging ring's bytes");
 // the staging ring (or the mean mode's column), then czb, cza, czg of levels 0 .. nz+1
-template <typename C>
-__host__ __device__ constexpr size_t tri_coef_off(int nz) {
-  return ((TRI_SMEM > (size_t)nz * sizeof(C) ? TRI_SMEM : (size_t)nz * sizeof(C)) + 15) & ~(size_t)15;
-}
-template <typename C>
-static size_t tri_smem_bytes(int nz) { return tri_coef_off<C>(nz) + 3 * (size_t)(nz + 2) * sizeof(double); }
+static size_t tri_smem_bytes(int nz) { return TRI_SMEM + 3 * (size_t)(nz + 2) * sizeof(double); }
 constexpr size_t TRI_SMEM_MAX = TRI_SMEM + 3 * (size_t)(MGPU_MAX_NZ + 2) * sizeof(double);
 template <typename T>
 __global__ void k_tridiag(typename Cx<T>::t* __restrict__ spec, double2* __restrict__ s1buf, const double* __restrict__ b1,
                           const double* __restrict__ prof, int prof_stride, int nx, int ny, int nz, int transpose,
                           int ncols, int kx0, int rpb);
-// the staging buffers exceed the default 48 KB of dynamic shared memory: raise the limit once per
-// device (the largest column, nz = MGPU_MAX_NZ levels for the mean mode, stays below TRI_SMEM)
+// the staging buffers exceed the default 48 KB of dynamic shared memory: raise the limit once per device
 static void ensure_tri_attr() {
   static std::mutex mu;
   static bool done[64] = {};
@@ -1094,7 +1091,6 @@ __device__ __forceinline__ unsigned char* tri_smem() {
 // recurrence waits for a multiply-add per level: with the divisions in the recurrence and its operands
 // loaded in turn, this block was the last to finish and set the time of the whole solve (21 of 21 us at
 // 64 x 64 x 65, 31 at 128 x 128 x 96, 41 of 46 at 256 x 256 x 128, FP64).  smem: mean_smem(nz) bytes.
-__host__ __device__ constexpr size_t mean_smem(int nz) { return (size_t)(nz + 2) * (sizeof(double2) + 2 * sizeof(double)); }
 template <typename T>
 __device__ void mean_mode_block(typename Cx<T>::t* sp, long long lstride, int nz, const double* __restrict__ prof,
                                 int prof_stride, int transpose, unsigned char* smem) {
@@ -1158,7 +1154,7 @@ __global__ void k_tridiag(typename Cx<T>::t* __restrict__ spec, double2* __restr
   const long long lstride = (long long)rpb * ncols;   // level stride of the spectrum
   // the three coefficient profiles, read at every level of every column, from shared memory
   const int cs = nz + 2;
-  double* cf = reinterpret_cast<double*>(tri_smem() + tri_coef_off<C>(nz));
+  double* cf = reinterpret_cast<double*>(tri_smem() + TRI_SMEM);
   for (int q = threadIdx.x; q < 3 * cs; q += blockDim.x) {
     const int r = q / cs, kk = q - r * cs;
     cf[q] = prof[(r == 0 ? P_CZB : (r == 1 ? P_CZA : P_CZG)) * prof_stride + kk];
@@ -1394,13 +1390,17 @@ __global__ void __launch_bounds__(SEG_COLS * SEG_MAX) k_tridiag_seg(typename Cx<
 }
 
 // Segmented solve or one thread per column?  Columns for fewer than four blocks of 32 per SM, on up
-// to 193 levels (SEG_MAX segments of 12), are too few for the column
-// kernel (64 x 64 x 65 in FP64 4.5 us against 14.2, 128 x 128 x 96 10.5 against 21.6; but 256 x 256 x 128 39.8
-// against 33.5, where the column kernel streams).  The whole grid's
-// columns decide, so that a y-slab's block of them is solved as the single domain solves it.
+// to 193 levels (SEG_MAX segments of 12), are too few for the column kernel.  Segments against columns
+// (the stage with its events), FP64 and FP32: 64 x 64 x 65 9.2 and 18.4, 9.4 and 20.3 us; 64 x 64 x 193 14.3 and
+// 45.0, 14.3 and 47.1; 192 x 192 x 64 16.3 and 22.4, 15.0 and 22.6; 256 x 144 x 129 26.8 and 37.3, 26.2 and 38.9.
+// Beyond the line the column kernel streams: 256 x 256 x 128 43.1 and 37.9, 38.9 and 40.9; 512 x 512 x 160 276 and 220,
+// 224 and 207 (in FP32 segments still win on fewer levels: 512 x 512 x 40 36.7 and 55.3).  The whole grid's
+// columns decide, so that a y-slab's block of them is solved as the single domain solves it, and for the same
+// reason the 148 SMs of a B200 are a constant.
+constexpr long long SEG_SMS = 148;
 static int seg_levels(long long columns, int nz) {
   const int rows = nz - 1;
-  if (columns > 148LL * 4 * SEG_COLS || rows > 12 * SEG_MAX) return 0;
+  if (columns > SEG_SMS * 4 * SEG_COLS || rows > 12 * SEG_MAX) return 0;
   return rows <= 4 * SEG_MAX ? 4 : (rows <= 8 * SEG_MAX ? 8 : 12);
 }
 template <typename T>
@@ -1424,11 +1424,10 @@ static bool launch_tridiag_seg(typename Cx<T>::t* spec, const double* b1, const 
 template <typename T>
 static void launch_tridiag(typename Cx<T>::t* spec, double2* s1, const double* b1, const double* prof, int prof_stride,
                            int nx, int ny, int nz, bool transpose, int ncols, int kx0, int rpb, cudaStream_t st) {
-  typedef typename Cx<T>::t C;
   const long long ncol = (long long)ny * ncols;
   if (launch_tridiag_seg<T>(spec, b1, prof, prof_stride, nx, ny, nz, transpose, ncols, kx0, rpb, st)) return;
   ensure_tri_attr();
-  k_tridiag<T><<<(unsigned)((ncol + TRI_TB - 1) / TRI_TB + (kx0 == 0 ? 1 : 0)), TRI_TB, tri_smem_bytes<C>(nz), st>>>(
+  k_tridiag<T><<<(unsigned)((ncol + TRI_TB - 1) / TRI_TB + (kx0 == 0 ? 1 : 0)), TRI_TB, tri_smem_bytes(nz), st>>>(
       spec, s1, b1, prof, prof_stride, nx, ny, nz, transpose ? 1 : 0, ncols, kx0, rpb);
 }
 

@@ -38,7 +38,7 @@ enum { L_T1, L_T2, L_D1, L_D2, L_RDZ, L_RDZN, L_GWX, L_GWY, L_N };  // level con
 constexpr int RL = 4;
 // levels k, k+1 and the one in flight; vis also k-1
 constexpr int RP = 3, RVIS = 4;
-template <typename T, bool TVD>
+template <typename T>
 constexpr size_t smem_bytes() {
   return sizeof(T) * ((size_t)(6 * RP + RVIS) * G<T>::PLANE + (size_t)RL * L_N + (size_t)10 * CN);
 }
@@ -333,7 +333,7 @@ __global__ void __launch_bounds__(NT, ctas<T>()) k_f_momentum(const __grid_const
 
 template <typename T>
 static int launch(const Scalars& s, DevState<T>& d, cudaStream_t st) {
-  const size_t smem = smem_bytes<T, false>();
+  const size_t smem = smem_bytes<T>();
   static LaunchTable table;
   const LaunchLimits lim =
       launch_limits(table, {(const void*)k_f_momentum<T, false>, (const void*)k_f_momentum<T, true>}, NT, smem);

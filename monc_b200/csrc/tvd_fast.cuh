@@ -563,6 +563,8 @@ __global__ void __launch_bounds__(NT, ctas<T, NS, DIM>()) k_f_tvd(const __grid_c
       }
       // what of the source needs the planes: diffusion, damping, subsidence
       T src[NS], zv[NS];
+#pragma unroll
+      for (int n = 0; n < NS; ++n) src[n] = (T)0.0;
       auto local_source = [&]() {
         if (job.first && s.th_baroclinic) src[0] = src[0] + ((v0 + (T)s.vgal) * (T)s.mfx - (u0 + (T)s.ugal) * (T)s.mfy);
         if (s.use_vd) {
@@ -602,8 +604,6 @@ __global__ void __launch_bounds__(NT, ctas<T, NS, DIM>()) k_f_tvd(const __grid_c
           }
         }
       };
-#pragma unroll
-      for (int n = 0; n < NS; ++n) src[n] = (T)0.0;
       if constexpr (DB && DIM < 0) local_source();
       if constexpr (DB) asm volatile("cp.async.wait_all;\n" ::: "memory");
       __syncthreads();
