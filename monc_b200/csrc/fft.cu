@@ -450,12 +450,12 @@ __global__ void __launch_bounds__(line_block(LOGN)) k_fft_y(typename Cx<T>::t* _
 // result in natural order.
 //
 // Radices go up to 10, composite ones built in registers, so that most lengths take two or three
-// passes (360 = 6 6 10; 12, 15 and 16 would need more registers than two blocks per SM leave; the passes of radix 4, 2, 3 and 5 these replace were five, each with a
-// barrier, a division per point and its own twiddle loads); a block holds as many lines as give its
-// threads one butterfly each.  360 x 300 x 81, FP64: x forward with the pressure source, a kernel of
+// passes (360 = 6 6 10; 12, 15 and 16 would need more registers than two blocks per SM leave; the passes
+// of radix 4, 2, 3 and 5 these replace were five, each with a barrier, a division per point and its own
+// twiddle loads); a block holds as many lines as give its threads one butterfly each.  360 x 300 x 81, FP64: x forward with the pressure source, a kernel of
 // its own before, 0.058 + 0.146 -> 0.115, y 0.190 + 0.176 -> 0.098 + 0.094, x inverse 0.142 -> 0.076 ms
-// (the bytes of a transform take 0.021 ms; some 220 instructions per point at a quarter of the issue
-// slots with 16 warps per SM).  Radices up to 6 without spills: 0.124, 0.115 + 0.109, 0.089.
+// (the bytes of a transform take 0.021 ms; with 16 warps per SM they wait for memory, at a third of the issue
+// slots and 57 .. 66% of the shared-memory pipe).  Radices up to 6 without spills: 0.124, 0.115 + 0.109, 0.089.
 struct GenPlan {
   int n = 0, npass = 0;
   int lines = 0, block = 0;  // lines per block (a power of two) and threads per block

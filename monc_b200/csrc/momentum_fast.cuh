@@ -15,8 +15,9 @@
 //    with two barriers a level).
 // 256 x 256 x 128: FP64 0.275 -> 0.246 ms (738 MB, 0.113 ms), FP32 0.170 -> 0.151 ms; moist
 // 512 x 512 x 160: 1.78 -> 1.15 and 1.02 -> 0.71 ms; 1024 x 1024 x 200 with five q fields, FP32:
-// 7.07 -> 3.40 ms.  What is left is latency with 16 warps per SM (128 registers, 90 KB): copies in
-// flight, shared-memory loads and a barrier a level.
+// 7.07 -> 3.40 ms.  What is left in FP64 is latency with 16 warps per SM (128 registers, 90 KB): copies in
+// flight, shared-memory loads and a barrier a level (45% of the issue slots, 58% of the shared-memory
+// pipe); FP32 issues in 86% of its slots.
 // Sizes that no tile divides run here too: 360 x 300 x 81 in FP64 took 1.67 ms in the point kernel
 // for momentum and theta, now 0.28 and 0.28 ms.
 #pragma once

@@ -9,8 +9,9 @@
 // level ahead with cp.async.  Sizes that no tile divides are allowed: the staged planes wrap
 // periodically past the domain's edge and the columns beyond it are computed and not stored.
 //
-// What bounds it is instruction issue, so the face formulas (ultimateflux.F90) are arranged for few
-// instructions and are equal to tvd_face_x/y/z of dycore_device.cuh to rounding:
+// What bounds it is instruction issue (FP32: 88% of the slots) and in FP64, with 16 warps per SM, the
+// shared-memory pipe (71%, three fields 60%; 56% of the issue slots), so the face formulas (ultimateflux.F90)
+// are arranged for few instructions and are equal to tvd_face_x/y/z of dycore_device.cuh to rounding:
 //  * upwind values are addressed, not selected: the sign of the velocity picks the upwind cell and
 //    a direction, and three loads give fu, fc, fd;
 //  * the limiter is taken on magnitudes relative to fc (see limit), without a division by fd - fu
@@ -24,7 +25,7 @@
 // 256 x 256 x 128 0.373 -> 0.246 ms in FP64 and 0.250 -> 0.162 ms in FP32; theta, vapour and liquid
 // at 512 x 512 x 160 5.78 -> 2.54 and 3.47 -> 1.35 ms; theta and five q fields at 1024 x 1024 x 200
 // in FP32 36.6 -> 12.2 ms; u, v, w at 256 x 256 x 128 in FP64 1.12 -> 0.64 ms.  FP64 moves 537 MB
-// for theta, 0.082 ms; what is left above that is issue and latency with 16 warps per SM.
+// for theta, 0.082 ms.
 #pragma once
 
 #include "reciprocal.cuh"
