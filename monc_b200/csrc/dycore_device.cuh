@@ -247,6 +247,10 @@ __device__ T moist_ri(const Scalars& s, const PA& P, T ssq, const A& TH, const A
   else return scltmp * tmpinv * ((T)s.thconb * (qt_kp1 - qt_k) + ((thvln - thvli) - (thvun - thvui)) * (T)s.repsh);
 }
 
+// The moist Richardson number needs the vapour and liquid fields; with fewer q fields (and none is set in
+// the accessors then) the dry one is taken.
+__device__ __forceinline__ bool moist_richardson(const Scalars& s) { return !s.passive_q && s.nq > 1; }
+
 // vis/diff at level 2 <= k <= nz-1 from the strain rate and Richardson number
 template <typename T, class PA, class ATC, class AT>
 __device__ void smagorinsky_from_strain(const Scalars& s, const PA& P, T ssq, const ATC& THcur, const AT& THarg,
@@ -259,7 +263,7 @@ __device__ void smagorinsky_from_strain(const Scalars& s, const PA& P, T ssq, co
   // have one sign); the values agree to rounding.
   T X = (T)0.0;
   if (!s.passive_th) {
-    if (!s.passive_q) X = moist_ri<T, AT, PA, true>(s, P, ssq, THarg, *QV, *QL, k, j, i);
+    if (moist_richardson(s)) X = moist_ri<T, AT, PA, true>(s, P, ssq, THarg, *QV, *QL, k, j, i);
     else X = (P(P_DTHREF, k) + THcur(k + 1, j, i) - THcur(k, j, i)) * P(P_RDZN, k + 1) * P(P_BUOY_CO, k);
   }
   const T rn = P(P_RNEUTML_SQ, k);
@@ -283,7 +287,7 @@ __device__ void smagorinsky_from_strain(const Scalars& s, const PA& P, T ssq, co
 #else
   T ri = (T)0.0;
   if (!s.passive_th) {
-    if (!s.passive_q) ri = moist_ri<T, AT>(s, P, ssq, THarg, *QV, *QL, k, j, i);
+    if (moist_richardson(s)) ri = moist_ri<T, AT>(s, P, ssq, THarg, *QV, *QL, k, j, i);
     else  // the dry branch reads current_state%th in both stepping modes
       ri = (P(P_DTHREF, k) + THcur(k + 1, j, i) - THcur(k, j, i)) * P(P_RDZN, k + 1) * P(P_BUOY_CO, k) / ssq;
   }

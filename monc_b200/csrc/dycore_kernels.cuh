@@ -104,7 +104,7 @@ __global__ void k_c_smagorinsky(Scalars s, DevState<T> d) {
   View<T> U = view<T>(fwd ? d.u : d.zu, s), V = view<T>(fwd ? d.v : d.zv, s), W = view<T>(fwd ? d.w : d.zw, s);
   View<T> THc = view<T>(d.th, s), THa = view<T>(fwd ? d.th : d.zth, s);
   View<T> QV, QL;
-  if (!s.passive_q && s.nq > 1) {
+  if (moist_richardson(s)) {
     QV = view<T>(fwd ? d.q[s.iqv] : d.zq[s.iqv], s);
     QL = view<T>(fwd ? d.q[s.iql] : d.zq[s.iql], s);
   }
@@ -559,7 +559,7 @@ __global__ void k_f_subgrid(Scalars s, DevState<T> d) {
   if (k == s.nz) { d.vis[o] = (T)0.0; d.diff[o] = (T)0.0; return; }
   View<T> U = view<T>(fwd ? d.u : d.zu, s), V = view<T>(fwd ? d.v : d.zv, s), W = view<T>(fwd ? d.w : d.zw, s);
   View<T> QV, QL;
-  if (!s.passive_q && s.nq > 1) {
+  if (moist_richardson(s)) {
     QV = view<T>(fwd ? d.q[s.iqv] : d.zq[s.iqv], s);
     QL = view<T>(fwd ? d.q[s.iql] : d.zq[s.iql], s);
   }
@@ -1546,7 +1546,7 @@ __global__ void __launch_bounds__(tiled::NT, tiled::ctas_scalar<T>()) k_f_smag_t
     for (int kk = kb - 1; kk <= kb + 2 && kk <= nz; ++kk) rP[(kk & (RP - 1)) * P_COUNT + tid] = load_profile<T>(s, tid, kk);
   const View<T> THc = view<T>(d.th, s), THa = view<T>(fwd ? d.th : d.zth, s);
   View<T> QV, QL;
-  const bool moist = !s.passive_q && s.nq > 1;
+  const bool moist = moist_richardson(s);
   if (moist) {
     QV = view<T>(fwd ? d.q[s.iqv] : d.zq[s.iqv], s);
     QL = view<T>(fwd ? d.q[s.iql] : d.zq[s.iql], s);
